@@ -850,6 +850,9 @@ namespace lible_b200
             a.mode = kStore;
             a.out = d_out;
             LaunchFn fn = lookupFwd64(swap ? tk : tb, swap ? tb : tk);
+            if (splitStore(bra, ket, n) && !splitFlipped(swap ? tk : tb, swap ? tb : tk, false))
+                if (const LaunchFn sf = lookupSplit(swap ? tk : tb, swap ? tb : tk, false))
+                    fn = sf;
             if (!fn)
                 throw EngineError(kStatusUnsupported, "quartet class not instantiated");
             cudaCheck(fn(a, stream_, num_sms_), "eri kernel");
@@ -1319,7 +1322,7 @@ namespace lible_b200
     }
 
     Engine::JKClassPair Engine::buildClassPair(const ClassSet &bs, int cb, const ClassSet &ks, int ck, bool triangle,
-                                               double thr, double thr32, bool mixed)
+                                               double thr, double thr32, bool mixed, bool split)
     {
         const ClassOrder &ob = bs.orders[cb], &ok = ks.orders[ck];
         // survivors of the predicate q_b * qj >= t in a group: a prefix of its Q values in decreasing
@@ -1334,6 +1337,7 @@ namespace lible_b200
         JKClassPair cp;
         cp.cb = cb;
         cp.ck = ck;
+        cp.split = split;
         cp.all64 = mixed && fp32InFp64(bs.host[cb].la, bs.host[cb].lb, ks.host[ck].la, ks.host[ck].lb);
         if (cp.all64)
             mixed = false;  // one FP64 task sequence over every surviving quartet
@@ -1463,6 +1467,45 @@ namespace lible_b200
         return cp;
     }
 
+    // Number of leading runs (heaviest first) of a register-path launch whose quartets are split over
+    // the thread groups of a warp.  A quartet's primitive pairs are otherwise one thread group's serial
+    // chain (64 x 64 pairs of two contracted core pairs: about 1.6 ms of (ss|ss) on an otherwise idle
+    // device), so a launch cannot end before the chain of its heaviest quartet.  Split are the
+    // quartets with at least as many pairs as every resident group (16 warps per SM) gets when the
+    // launch is spread evenly, and at least 32 (8 when every quartet can have a warp of its own): with
+    // fewer the reduction and the digestion by one quartet cost more than the chain.  Measured: (ss|ss)
+    // of (H2O)_16 cc-pVDZ 2.64 -> 1.56 ms, of one water 1.61 -> 0.10 ms; with the finer chunks and 16
+    // streams of small plans the whole J/K of one water went from 2.38 to 0.25 ms, of (H2O)_5 def2-SVP
+    // from 1.38 to 0.76 ms.  Splitting from half or a quarter of the even share on slows the classes that
+    // fill the device anyway ((dp|ss) of (H2O)_16 0.89 -> 0.99 ms), from 14 pairs on the (H2O)_5 build
+    // (1.21 ms).
+    static size_t splitRuns(const std::vector<unsigned long long> &n, const std::vector<double> &c, int unit, int num_sms)
+    {
+        double total = 0;
+        unsigned long long tasks = 0;
+        for (size_t i = 0; i < n.size(); i++)
+        {
+            total += (double)n[i] * c[i];
+            tasks += n[i];
+        }
+        const double warps = 16.0 * num_sms;
+        const double limit = std::max((double)tasks <= warps ? 8.0 : 32.0, total / (warps * std::max(unit, 1)));
+        size_t lead = 0;
+        while (lead < n.size() && c[lead] >= limit)
+            lead++;
+        return lead;
+    }
+
+    // Store launches take explicit lists whose contraction lengths the host does not look at: every
+    // quartet is split when the class averages at least 4 primitive pairs per quartet and the list
+    // would not give each warp slot of the device (16 per SM) 8 quartets.
+    bool Engine::splitStore(const DevPairClass &bra, const DevPairClass &ket, long long n) const
+    {
+        const double k = (double)bra.n_ppairs / std::max<size_t>(bra.n_pairs, 1) * (double)ket.n_ppairs /
+                         std::max<size_t>(ket.n_pairs, 1);
+        return k >= 4.0 && n < 8LL * 16 * num_sms_;
+    }
+
     // (Re)cuts the FP64 or FP32 task sequence of a class pair into work-queue chunks of at most
     // `mult` work units.
     void Engine::rebuildChunks(JKClassPair &cp, bool fp32, int mult)
@@ -1480,7 +1523,20 @@ namespace lible_b200
         const int unit = unitFwd(tb, tk, fp32, fp32 ? cp.shape32 : cp.shape64);
         if (unit == 0)
             return;
-        auto ch = costChunks(fp32 ? cp.run32 : cp.run64, cp.cost, unit, mult * unit);
+        // a launch with few tasks is cut finer, down to one worker step a chunk, so that its chunks reach
+        // every resident worker (16 warps, or as many blocks, per SM)
+        mult = (int)std::min<long long>(mult, std::max<long long>(1, n / (16LL * num_sms_ * unit)));
+        const auto &runs = fp32 ? cp.run32 : cp.run64;
+        const size_t lead = cp.split && lookupSplit(tb, tk, fp32) ? splitRuns(runs, cp.cost, unit, num_sms_) : 0;
+        // the split launch's chunks first (runs come heaviest first), one to four tasks each
+        auto ch = costChunks({runs.begin(), runs.begin() + lead}, {cp.cost.begin(), cp.cost.begin() + lead}, 1,
+                             mult > 1 ? 4 : 1);
+        (fp32 ? cp.n_split32 : cp.n_split64) = (long long)ch.size() - 1;
+        const auto rest =
+            costChunks({runs.begin() + lead, runs.end()}, {cp.cost.begin() + lead, cp.cost.end()}, unit, mult * unit);
+        const unsigned long long base = ch.back();
+        for (size_t i = 1; i < rest.size(); i++)
+            ch.push_back(base + rest[i]);
         (fp32 ? cp.n_chunks32 : cp.n_chunks64) = (long long)ch.size() - 1;
         dev = devUpload(ch, stream_);
     }
@@ -1500,7 +1556,7 @@ namespace lible_b200
         for (size_t cb = 0; cb < nc; cb++)
             for (size_t ck = 0; ck <= cb; ck++)
             {
-                JKClassPair cp = buildClassPair(cs, (int)cb, cs, (int)ck, cb == ck, thr, thr32, mixed);
+                JKClassPair cp = buildClassPair(cs, (int)cb, cs, (int)ck, cb == ck, thr, thr32, mixed, true);
                 if (cp.n64 + cp.n32 == 0)
                     continue;
                 plan.n_quartets += cp.n64 + cp.n32;
@@ -1514,7 +1570,7 @@ namespace lible_b200
         std::stable_sort(plan.pairs.begin(), plan.pairs.end(), [](const JKClassPair &x, const JKClassPair &y) {
             return x.flops64 + x.flops32 > y.flops64 + y.flops32;
         });
-        plan.counters = devAlloc<unsigned long long>(2 * std::max<size_t>(plan.pairs.size(), 1));
+        plan.counters = devAlloc<unsigned long long>(4 * std::max<size_t>(plan.pairs.size(), 1));
         plan.key = key;
         applyTuneCache(plan);
         assignBranches(plan);
@@ -1530,10 +1586,14 @@ namespace lible_b200
     void Engine::assignBranches(JKPlan &plan)
     {
         double load[kBranches] = {};
+        // a small build's launches each leave most of the device idle and last as long as their longest
+        // quartet, so they run side by side on all streams; launches that fill the device gain nothing
+        // from more than four
+        const int nb = plan.flops64 + 0.5 * plan.flops32 < 2e10 ? kBranches : 4;
         for (auto &cp : plan.pairs)
         {
             int b = 0;
-            for (int i = 1; i < kBranches; i++)
+            for (int i = 1; i < nb; i++)
                 if (load[i] < load[b])
                     b = i;
             cp.branch = b;
@@ -1600,16 +1660,97 @@ namespace lible_b200
         a.ket_EtP = bra_etp;
     }
 
+    // Arguments of the FP64 or FP32 class launch of plan entry `ip` (its whole task sequence; the split
+    // and the ordinary launch each take their part of the chunks).
+    QuartetArgs Engine::jkArgs(const JKPlan &plan, size_t ip, bool fp32, bool mixed, const double *D, double *J, double *K)
+    {
+        ClassSet &cs = mainSet(true);
+        const auto &cp = plan.pairs[ip];
+        const auto &B = cs.dev[cp.cb], &Kc = cs.dev[cp.ck];
+        QuartetArgs a{};
+        a.bra = view(B);
+        a.ket = view(Kc);
+        a.boys = boys_;
+        a.boys_f = boys_f_;
+        a.major_ket = 1;
+        a.major_order = cp.majors;
+        a.minor_order = cs.orders[cp.cb].d_order;
+        a.n_major = cp.n_bra;
+        a.same_class = cp.cb == cp.ck;
+        a.mode = kJK;
+        a.D = D;
+        a.J = J;
+        a.K = K;
+        a.nao = (int)nao_;
+        a.n_tasks = fp32 ? cp.t32 : cp.t64;
+        a.prefix = fp32 ? cp.prefix32 : cp.prefix64;
+        a.minor_begin = fp32 ? cp.begin32 : cp.begin64;
+        a.chunks = (fp32 ? cp.chunks32 : cp.chunks64) + (fp32 ? cp.n_split32 : cp.n_split64);
+        a.n_chunks = fp32 ? cp.n_chunks32 - cp.n_split32 : cp.n_chunks64 - cp.n_split64;
+        a.counter = plan.counters + 2 * ip + (fp32 ? 1 : 0);
+        a.grid_div = fp32 ? cp.grid_div32 : cp.grid_div64;
+        a.bra_qpos = cs.orders[cp.cb].d_q;
+        a.bra_qpair = B.Q;
+        a.ket_qpair = Kc.Q;
+        a.q_lo = fp32 ? plan.thr : ((mixed && !cp.all64) ? plan.thr32 : plan.thr);
+        a.q_hi = fp32 ? plan.thr32 : HUGE_VAL;
+        a.bra_soa = B.soa;
+        a.bra_pPs = B.pPs;
+        a.bra_Es = B.Es;
+        a.bra_Efs = B.Efs;
+        a.bra_pPfs = B.pPfs;
+        a.bra_soa2 = B.soa2;
+        a.bra_Dab = B.Dab;
+        a.bra_npos = (int)B.n_pairs;
+        a.ket_EtP = Kc.EtP;
+        a.status = d_status_;
+        return a;
+    }
+
+    // The split launch of plan entry `ip` (its heavily contracted quartets; none: no launch).
+    void Engine::launchSplitJK(const JKPlan &plan, size_t ip, bool fp32, bool mixed, const double *D, double *J, double *K,
+                               cudaStream_t st)
+    {
+        const auto &cp = plan.pairs[ip];
+        const long long n = fp32 ? cp.n_split32 : cp.n_split64;
+        if (n == 0)
+            return;
+        QuartetArgs a = jkArgs(plan, ip, fp32, mixed, D, J, K);
+        a.chunks -= n;
+        a.n_chunks = n;
+        a.counter += 2 * plan.pairs.size();
+        if (splitFlipped(cp.tb, cp.tk, fp32))
+            flipOrientation(a, mainSet(true).dev[cp.cb].EtP);
+        cudaCheck(lookupSplit(cp.tb, cp.tk, fp32)(a, st, num_sms_), "jk split kernel");
+    }
+
+    // The ordinary launch of plan entry `ip`.
+    void Engine::launchClassJK(const JKPlan &plan, size_t ip, bool fp32, bool mixed, const double *D, double *J, double *K,
+                               cudaStream_t st)
+    {
+        const auto &cp = plan.pairs[ip];
+        const int shape = fp32 ? cp.shape32 : cp.shape64;
+        const LaunchFn fn = fp32 ? lookupFwd32(cp.tb, cp.tk, shape) : lookupFwd64(cp.tb, cp.tk, shape);
+        if (!fn)
+            throw EngineError(kStatusUnsupported, fp32 ? "FP32 quartet class not instantiated" : "quartet class not instantiated");
+        QuartetArgs a = jkArgs(plan, ip, fp32, mixed, D, J, K);
+        if (a.n_chunks <= 0)
+            return;
+        if (shape == 2)
+            flipOrientation(a, mainSet(true).dev[cp.cb].EtP);
+        cudaCheck(fn(a, st, num_sms_), fp32 ? "jk kernel fp32" : "jk kernel");
+    }
+
     // Launches one J/K build of `plan` (memsets, class kernels over the stream branches, block
     // symmetrisation) on stream_; usable inside a stream capture.  With a timer every class launch
     // goes to stream_ itself, bracketed by events.
     void Engine::enqueueJK(JKPlan &plan, const double *D, double *J, double *K, bool mixed, LaunchTimer *timer)
     {
-        ClassSet &cs = mainSet(true);
+        const ClassSet &cs = mainSet(true);
         const size_t n = (size_t)packed_;
         cudaCheck(cudaMemsetAsync(J, 0, n * sizeof(double), stream_), "memset");
         cudaCheck(cudaMemsetAsync(K, 0, n * sizeof(double), stream_), "memset");
-        cudaCheck(cudaMemsetAsync(plan.counters, 0, 2 * plan.pairs.size() * sizeof(unsigned long long), stream_),
+        cudaCheck(cudaMemsetAsync(plan.counters, 0, 4 * plan.pairs.size() * sizeof(unsigned long long), stream_),
                   "memset");
         gatherDab(D);
         cudaCheck(cudaMemsetAsync(d_status_, 0, sizeof(int), stream_), "memset");
@@ -1621,89 +1762,31 @@ namespace lible_b200
         for (int b = 0; b < kBranches; b++)
             if (used[b])
                 cudaCheck(cudaStreamWaitEvent(branch_[b], fork_, 0), "fork");
+        // the split launches of every class first: their quartets are the longest
+        if (!timer)
+            for (size_t ip = 0; ip < plan.pairs.size(); ip++)
+                for (int fp32 = 0; fp32 < (mixed ? 2 : 1); fp32++)
+                    launchSplitJK(plan, ip, fp32 == 1, mixed, D, J, K, branch_[plan.pairs[ip].branch]);
         for (size_t ip = 0; ip < plan.pairs.size(); ip++)
         {
             const auto &cp = plan.pairs[ip];
-            const auto &B = cs.dev[cp.cb], &Kc = cs.dev[cp.ck];
-            cudaStream_t st = timer ? stream_ : branch_[cp.branch];
             const auto &Bh = cs.host[cp.cb], &Kh = cs.host[cp.ck];
-            QuartetArgs a{};
-            a.bra = view(B);
-            a.ket = view(Kc);
-            a.boys = boys_;
-            a.boys_f = boys_f_;
-            a.list = nullptr;
-            a.major_ket = 1;
-            a.major_order = cp.majors;
-            a.minor_order = cs.orders[cp.cb].d_order;
-            a.n_major = cp.n_bra;
-            a.same_class = cp.cb == cp.ck;
-            a.mode = kJK;
-            a.D = D;
-            a.J = J;
-            a.K = K;
-            a.nao = (int)nao_;
-            a.n_tasks = cp.t64;
-            a.prefix = cp.prefix64;
-            a.minor_begin = cp.begin64;
-            a.chunks = cp.chunks64;
-            a.n_chunks = cp.n_chunks64;
-            a.counter = plan.counters + 2 * ip;
-            a.grid_div = cp.grid_div64;
-            a.bra_qpos = cs.orders[cp.cb].d_q;
-            a.bra_qpair = B.Q;
-            a.ket_qpair = Kc.Q;
-            a.q_lo = (mixed && !cp.all64) ? plan.thr32 : plan.thr;
-            a.q_hi = HUGE_VAL;
-            a.bra_soa = B.soa;
-            a.bra_pPs = B.pPs;
-            a.bra_Es = B.Es;
-            a.bra_Efs = B.Efs;
-            a.bra_pPfs = B.pPfs;
-            a.bra_soa2 = B.soa2;
-            a.bra_Dab = B.Dab;
-            a.bra_npos = (int)B.n_pairs;
-            a.ket_EtP = Kc.EtP;
-            a.status = d_status_;
-            LaunchFn f64 = lookupFwd64(cp.tb, cp.tk, cp.shape64);
-            if (!f64)
-                throw EngineError(kStatusUnsupported, "quartet class not instantiated");
-            if (timer && cp.t64 > 0)
+            for (int fp32 = 0; fp32 < (mixed ? 2 : 1); fp32++)
             {
-                timer->before(st);
-                timer->info.push_back({{Bh.la, Bh.lb, Kh.la, Kh.lb}, 2 * cp.shape64, 0.0, cp.flops64, cp.n64});
-            }
-            {
-                QuartetArgs a64 = a;
-                if (cp.shape64 == 2)
-                    flipOrientation(a64, B.EtP);
-                cudaCheck(f64(a64, st, num_sms_), "jk kernel");
-            }
-            if (timer && cp.t64 > 0)
-                timer->after(st);
-            if (mixed && cp.t32 > 0)
-            {
-                a.q_lo = plan.thr;
-                a.q_hi = plan.thr32;
-                a.n_tasks = cp.t32;
-                a.prefix = cp.prefix32;
-                a.minor_begin = cp.begin32;
-                a.chunks = cp.chunks32;
-                a.n_chunks = cp.n_chunks32;
-                a.counter = plan.counters + 2 * ip + 1;
-                a.grid_div = cp.grid_div32;
-                LaunchFn f32 = lookupFwd32(cp.tb, cp.tk, cp.shape32);
-                if (!f32)
-                    throw EngineError(kStatusUnsupported, "FP32 quartet class not instantiated");
+                if ((fp32 ? cp.t32 : cp.t64) == 0)
+                    continue;
+                cudaStream_t st = timer ? stream_ : branch_[cp.branch];
                 if (timer)
                 {
                     timer->before(st);
-                    timer->info.push_back({{Bh.la, Bh.lb, Kh.la, Kh.lb}, 1 + 2 * cp.shape32, 0.0, cp.flops32, cp.n32});
+                    timer->info.push_back({{Bh.la, Bh.lb, Kh.la, Kh.lb},
+                                           fp32 + 2 * (fp32 ? cp.shape32 : cp.shape64),
+                                           0.0,
+                                           fp32 ? cp.flops32 : cp.flops64,
+                                           fp32 ? cp.n32 : cp.n64});
+                    launchSplitJK(plan, ip, fp32 == 1, mixed, D, J, K, st);
                 }
-                QuartetArgs a32 = a;
-                if (cp.shape32 == 2)
-                    flipOrientation(a32, B.EtP);
-                cudaCheck(f32(a32, st, num_sms_), "jk kernel fp32");
+                launchClassJK(plan, ip, fp32 == 1, mixed, D, J, K, st);
                 if (timer)
                     timer->after(st);
             }
@@ -1795,9 +1878,7 @@ namespace lible_b200
         {
             stats->n_quartets = plan.n_quartets;
             stats->n_fp32 = plan.n_fp32;
-            stats->n_launches = 2;
-            for (const auto &cp : plan.pairs)
-                stats->n_launches += 1 + (cp.t32 > 0 ? 1 : 0);
+            stats->n_launches = planLaunches(plan);
         }
     }
 
@@ -1885,7 +1966,7 @@ namespace lible_b200
         for (size_t ip = 0; ip < plan.pairs.size(); ip++)
         {
             JKClassPair &cp = plan.pairs[ip];
-            const auto &B = cs.dev[cp.cb], &Kc = cs.dev[cp.ck];
+            const auto &B = cs.dev[cp.cb];
             for (int fp32 = 0; fp32 < (mixed ? 2 : 1); fp32++)
             {
                 const long long n = fp32 ? cp.t32 : cp.t64;
@@ -1909,43 +1990,10 @@ namespace lible_b200
                     rebuildChunks(cp, fp32 == 1, cm);  // the work unit depends on the shape
                     for (int gd : grid_divs)
                     {
-                        QuartetArgs a{};
-                        a.bra = view(B);
-                        a.ket = view(Kc);
-                        a.boys = boys_;
-                        a.boys_f = boys_f_;
-                        a.major_ket = 1;
-                        a.major_order = cp.majors;
-                        a.minor_order = cs.orders[cp.cb].d_order;
-                        a.n_major = cp.n_bra;
-                        a.same_class = cp.cb == cp.ck;
-                        a.mode = kJK;
-                        a.D = D;
-                        a.J = J;
-                        a.K = K;
-                        a.nao = (int)nao_;
-                        a.n_tasks = n;
-                        a.prefix = fp32 ? cp.prefix32 : cp.prefix64;
-                        a.minor_begin = fp32 ? cp.begin32 : cp.begin64;
-                        a.chunks = fp32 ? cp.chunks32 : cp.chunks64;
-                        a.n_chunks = fp32 ? cp.n_chunks32 : cp.n_chunks64;
-                        a.counter = plan.counters + 2 * ip + fp32;
+                        QuartetArgs a = jkArgs(plan, ip, fp32 == 1, mixed, D, J, K);
+                        if (a.n_chunks <= 0)
+                            continue;  // every quartet in the split launch
                         a.grid_div = gd;
-                        a.bra_qpos = cs.orders[cp.cb].d_q;
-                        a.bra_qpair = B.Q;
-                        a.ket_qpair = Kc.Q;
-                        a.q_lo = fp32 ? plan.thr : ((mixed && !cp.all64) ? plan.thr32 : plan.thr);
-                        a.q_hi = fp32 ? plan.thr32 : HUGE_VAL;
-                        a.bra_soa = B.soa;
-                        a.bra_pPs = B.pPs;
-                        a.bra_Es = B.Es;
-                        a.bra_Efs = B.Efs;
-                        a.bra_pPfs = B.pPfs;
-                        a.bra_soa2 = B.soa2;
-                        a.bra_Dab = B.Dab;
-                        a.bra_npos = (int)B.n_pairs;
-                        a.ket_EtP = Kc.EtP;
-                        a.status = d_status_;
                         if (shape == 2)
                             flipOrientation(a, B.EtP);
                         // a second timing only for short launches, where one sample is noisy
@@ -2012,10 +2060,15 @@ namespace lible_b200
 
     long long Engine::jkLaunchCount(const JKOptions &opt)
     {
-        JKPlan &plan = jkPlan(opt.schwarz, opt.fp32_threshold, opt.precision == 1);
+        return planLaunches(jkPlan(opt.schwarz, opt.fp32_threshold, opt.precision == 1));
+    }
+
+    // Class and split kernels of one build, and the two symmetrisations.
+    long long Engine::planLaunches(const JKPlan &plan)
+    {
         long long c = 2;
         for (const auto &cp : plan.pairs)
-            c += 1 + (cp.t32 > 0 ? 1 : 0);
+            c += (cp.n_split64 > 0) + (cp.n_chunks64 > cp.n_split64) + (cp.n_split32 > 0) + (cp.n_chunks32 > cp.n_split32);
         return c;
     }
 

@@ -252,6 +252,7 @@ namespace lible_b200
             bool swap = false;  // RI plans: bra is the auxiliary class
             long long n64 = 0, n32 = 0;  // surviving quartets
             long long t64 = 0, t32 = 0;  // launched tasks (whole bra groups; the kernels test each)
+            bool split = false;          // heavily contracted quartets go to the class's split launch
             bool all64 = false;          // mixed plan, but every quartet of this pair in FP64
             double prim64 = 0, prim32 = 0, flops64 = 0, flops32 = 0;
             unsigned long long *prefix64 = nullptr, *prefix32 = nullptr;
@@ -259,6 +260,7 @@ namespace lible_b200
             // work-queue chunks (task boundaries) and the runs they are cut from
             unsigned long long *chunks64 = nullptr, *chunks32 = nullptr;
             long long n_chunks64 = 0, n_chunks32 = 0;
+            long long n_split64 = 0, n_split32 = 0;  // leading chunks of split (heavily contracted) quartets
             std::vector<unsigned long long> run64, run32;
             std::vector<double> cost;
             // launch parameters (autotuned): resident blocks per SM divided by grid_div, chunks of
@@ -284,15 +286,23 @@ namespace lible_b200
         // One class pair of a plan: bra class cb of set bs, ket class ck of set ks; `triangle`
         // keeps only unique pairs when both are the same class of the same set.
         JKClassPair buildClassPair(const ClassSet &bs, int cb, const ClassSet &ks, int ck, bool triangle,
-                                   double thr, double thr32, bool mixed);
+                                   double thr, double thr32, bool mixed, bool split = false);
         JKPlan &riPlan(double thr);
         JKPlan &ri2Plan(double thr);
         QuartetArgs riArgs(const JKPlan &plan, size_t ip);
         LaunchFn riLaunchFn(const JKPlan &plan, size_t ip);
 
         void rebuildChunks(JKClassPair &cp, bool fp32, int mult);
+        // Whether a store launch of n quartets of two classes splits every quartet over a warp.
+        bool splitStore(const DevPairClass &bra, const DevPairClass &ket, long long n) const;
         void assignBranches(JKPlan &plan);
         struct LaunchTimer;
+        QuartetArgs jkArgs(const JKPlan &plan, size_t ip, bool fp32, bool mixed, const double *D, double *J, double *K);
+        void launchSplitJK(const JKPlan &plan, size_t ip, bool fp32, bool mixed, const double *D, double *J, double *K,
+                           cudaStream_t st);
+        void launchClassJK(const JKPlan &plan, size_t ip, bool fp32, bool mixed, const double *D, double *J, double *K,
+                           cudaStream_t st);
+        static long long planLaunches(const JKPlan &plan);
         void enqueueJK(JKPlan &plan, const double *D, double *J, double *K, bool mixed, LaunchTimer *timer = nullptr);
         void gatherDab(const double *D);
         void applyTuneCache(JKPlan &plan);
@@ -327,7 +337,7 @@ namespace lible_b200
         int wait_inject_ = 0;  // see injectWaitTimeout
         double *staging_[4] = {};
         size_t staging_n_[4] = {};
-        static constexpr int kBranches = 4;
+        static constexpr int kBranches = 16;  // streams; a large plan uses the first four of them
         cudaStream_t branch_[kBranches] = {};
         cudaEvent_t fork_ = nullptr, join_[kBranches] = {};
         cudaGraphExec_t graph_exec_ = nullptr;

@@ -562,6 +562,26 @@ namespace lible_b200
         }
     }
 
+    // Grid dp x dq (dp dq <= parts, dp a power of two or `parts`) over which the ka x kq primitive pairs
+    // of one quartet are dealt out: the one with the fewest pairs per part, and of equals the one with
+    // the most bra parts (a lane then loads its bra records once and the ket's are broadcasts).
+    __device__ __forceinline__ void splitGrid(uint32_t ka, uint32_t kq, uint32_t parts, uint32_t &dp, uint32_t &dq)
+    {
+        uint32_t best = 0xffffffffu;
+        for (uint32_t x = 1;; x = 2 * x < parts ? 2 * x : parts)
+        {
+            const uint32_t y = parts / x, c = ((ka + x - 1) / x) * ((kq + y - 1) / y);
+            if (c <= best)
+            {
+                best = c;
+                dp = x;
+                dq = y;
+            }
+            if (x == parts)
+                break;
+        }
+    }
+
     // ---------------------------------------------------------------------------------------
     // Register path: a group of GT threads per contracted quartet, thread `member` owning the ket
     // columns [c0, c0 + CW) of the batch (c0 = member * CW).  Each thread evaluates the Boys
@@ -577,9 +597,13 @@ namespace lible_b200
     // `sv` is the bra's structure-of-arrays entry (sv.z = 0: read the per-pair records instead).
     // `nk` >= 0 is the bra's primitive-pair count from the per-position fields (the bra records are
     // then read from the structure-of-arrays copies only); -1 reads the pair's primitive range.
-    template <int LA, int LB, int LC, int LD, typename T, int SV = 0>
+    // SPLIT: this call sums part `part` of a quartet whose primitive pairs are dealt out in `parts`
+    // parts: the bra primitives sp, sp + dp, ... against the ket primitives sq, sq + dq, ... of the
+    // dp x dq grid of splitGrid (parts past the grid leave V at zero).
+    template <int LA, int LB, int LC, int LD, typename T, int SV = 0, bool SPLIT = false>
     __device__ __forceinline__ void quartetThread(const QuartetArgs &a, uint32_t ib, uint32_t ik, int c0, T *V,
-                                                  const T *btab, uint4 sv, int nk)
+                                                  const T *btab, uint4 sv, int nk, uint32_t part = 0,
+                                                  uint32_t parts = 1)
     {
         using C = Cls<LA, LB, LC, LD>;
         constexpr int CW = Shape<LA, LB, LC, LD, T, SV>::CW;
@@ -596,7 +620,16 @@ namespace lible_b200
         const T *Eb = braE<T>(a.bra);
         const T *Ek = ketE<T>(a.ket) + c0;
         const size_t sn = sv.z;
-        for (uint32_t p = p0; p < p1; p++)
+        uint32_t dp = 1, dq = 1, sp = 0, sq = 0;
+        if constexpr (SPLIT)
+        {
+            splitGrid(p1 - p0, q1 - q0, parts, dp, dq);
+            if (part >= dp * dq)
+                return;
+            sp = part % dp;
+            sq = part / dp;
+        }
+        for (uint32_t p = p0 + sp; p < p1; p += dp)
         {
             PQ4 P;          // FP64 record
             float Pf[8];    // FP32 record: p, 1/p, P hi, P lo
@@ -631,7 +664,7 @@ namespace lible_b200
 #pragma unroll
             for (int x = 0; x < C::HAB * CW; x++)
                 RxE[x] = T(0);
-            for (uint32_t q = q0; q < q1; q++)
+            for (uint32_t q = q0 + sq; q < q1; q += dq)
             {
                 T R[C::NR];
                 if constexpr (sizeof(T) == 8)

@@ -25,5 +25,9 @@ namespace lible_b200
     LaunchFn lookupFwd32(int bra_type, int ket_type, int shape = 0);
     LaunchFn lookupD1(int bra_type, int ket_type);
     int unitFwd(int bra_type, int ket_type, bool fp32, int shape = 0);
+    // Split form of a J/K or store class (null: none) and whether it runs the class in the other
+    // orientation, (cd|ab), because only that one takes the register path.
+    LaunchFn lookupSplit(int bra_type, int ket_type, bool fp32);
+    bool splitFlipped(int bra_type, int ket_type, bool fp32);
     bool hasFwdVariant(int bra_type, int ket_type, bool fp32, int shape = 1);
 }

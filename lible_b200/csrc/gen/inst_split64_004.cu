@@ -1,0 +1,28 @@
+// Generated by gen_instances.py: split forms of (2,1|1,1), (2,1|2,0), (2,1|2,1).
+#include "../eri_launch_fwd.cuh"
+#include "../eri_split_kernel.cuh"
+
+namespace lible_b200
+{
+    cudaError_t launch_split64_04_02(const QuartetArgs &a, cudaStream_t s, int n)
+    {
+        if constexpr (hasSplitForm<2,1,1,1,double>())
+            return launchSplit<2,1,1,1,double>(a, s, n);
+        else
+            return launchSplit<1,1,2,1,double>(a, s, n);
+    }
+    cudaError_t launch_split64_04_03(const QuartetArgs &a, cudaStream_t s, int n)
+    {
+        if constexpr (hasSplitForm<2,1,2,0,double>())
+            return launchSplit<2,1,2,0,double>(a, s, n);
+        else
+            return launchSplit<2,0,2,1,double>(a, s, n);
+    }
+    cudaError_t launch_split64_04_04(const QuartetArgs &a, cudaStream_t s, int n)
+    {
+        if constexpr (hasSplitForm<2,1,2,1,double>())
+            return launchSplit<2,1,2,1,double>(a, s, n);
+        else
+            return launchSplit<2,1,2,1,double>(a, s, n);
+    }
+}

@@ -1,5 +1,6 @@
 // Generated by gen_instances.py: lookup of class kernels.
 #include "../eri_launch_fwd.cuh"
+#include "../eri_split_kernel.cuh"
 
 namespace lible_b200
 {
@@ -637,6 +638,406 @@ namespace lible_b200
     static const LaunchFn k_d1_10[11] = {&launch_d1_10_00, &launch_d1_10_01, &launch_d1_10_02, &launch_d1_10_03, &launch_d1_10_04, &launch_d1_10_05, &launch_d1_10_06, &launch_d1_10_07, &launch_d1_10_08, &launch_d1_10_09, &launch_d1_10_10};
     static const LaunchFn k_d1_11[12] = {&launch_d1_11_00, &launch_d1_11_01, &launch_d1_11_02, &launch_d1_11_03, &launch_d1_11_04, &launch_d1_11_05, &launch_d1_11_06, &launch_d1_11_07, &launch_d1_11_08, &launch_d1_11_09, &launch_d1_11_10, &launch_d1_11_11};
     static const LaunchFn *const k_d1[12] = {k_d1_00, k_d1_01, k_d1_02, k_d1_03, k_d1_04, k_d1_05, k_d1_06, k_d1_07, k_d1_08, k_d1_09, k_d1_10, k_d1_11};
+    cudaError_t launch_split64_00_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_01_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_01_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_02_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_02_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_02_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_03_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_03_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_03_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_03_03(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_04_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_04_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_04_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_04_03(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_04_04(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_05_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_05_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_05_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_05_03(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_06_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_06_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_06_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_06_03(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_06_04(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_06_06(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_07_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_07_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_07_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_07_03(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_08_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_08_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split64_09_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_00_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_01_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_01_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_02_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_02_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_02_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_03_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_03_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_03_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_03_03(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_04_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_04_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_04_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_04_03(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_04_04(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_05_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_05_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_05_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_05_03(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_06_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_06_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_06_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_06_03(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_06_04(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_06_06(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_07_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_07_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_07_02(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_07_03(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_08_00(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_08_01(const QuartetArgs &, cudaStream_t, int);
+    cudaError_t launch_split32_09_00(const QuartetArgs &, cudaStream_t, int);
+    LaunchFn lookupSplit(int bt, int kt, bool fp32)
+    {
+        switch (100 * bt + kt)
+        {
+        case 0:
+            if (fp32)
+                return hasSplitForm<0,0,0,0,float>() || hasSplitForm<0,0,0,0,float>() ? &launch_split32_00_00 : nullptr;
+            else
+                return hasSplitForm<0,0,0,0,double>() || hasSplitForm<0,0,0,0,double>() ? &launch_split64_00_00 : nullptr;
+        case 100:
+            if (fp32)
+                return hasSplitForm<1,0,0,0,float>() || hasSplitForm<0,0,1,0,float>() ? &launch_split32_01_00 : nullptr;
+            else
+                return hasSplitForm<1,0,0,0,double>() || hasSplitForm<0,0,1,0,double>() ? &launch_split64_01_00 : nullptr;
+        case 101:
+            if (fp32)
+                return hasSplitForm<1,0,1,0,float>() || hasSplitForm<1,0,1,0,float>() ? &launch_split32_01_01 : nullptr;
+            else
+                return hasSplitForm<1,0,1,0,double>() || hasSplitForm<1,0,1,0,double>() ? &launch_split64_01_01 : nullptr;
+        case 200:
+            if (fp32)
+                return hasSplitForm<1,1,0,0,float>() || hasSplitForm<0,0,1,1,float>() ? &launch_split32_02_00 : nullptr;
+            else
+                return hasSplitForm<1,1,0,0,double>() || hasSplitForm<0,0,1,1,double>() ? &launch_split64_02_00 : nullptr;
+        case 201:
+            if (fp32)
+                return hasSplitForm<1,1,1,0,float>() || hasSplitForm<1,0,1,1,float>() ? &launch_split32_02_01 : nullptr;
+            else
+                return hasSplitForm<1,1,1,0,double>() || hasSplitForm<1,0,1,1,double>() ? &launch_split64_02_01 : nullptr;
+        case 202:
+            if (fp32)
+                return hasSplitForm<1,1,1,1,float>() || hasSplitForm<1,1,1,1,float>() ? &launch_split32_02_02 : nullptr;
+            else
+                return hasSplitForm<1,1,1,1,double>() || hasSplitForm<1,1,1,1,double>() ? &launch_split64_02_02 : nullptr;
+        case 300:
+            if (fp32)
+                return hasSplitForm<2,0,0,0,float>() || hasSplitForm<0,0,2,0,float>() ? &launch_split32_03_00 : nullptr;
+            else
+                return hasSplitForm<2,0,0,0,double>() || hasSplitForm<0,0,2,0,double>() ? &launch_split64_03_00 : nullptr;
+        case 301:
+            if (fp32)
+                return hasSplitForm<2,0,1,0,float>() || hasSplitForm<1,0,2,0,float>() ? &launch_split32_03_01 : nullptr;
+            else
+                return hasSplitForm<2,0,1,0,double>() || hasSplitForm<1,0,2,0,double>() ? &launch_split64_03_01 : nullptr;
+        case 302:
+            if (fp32)
+                return hasSplitForm<2,0,1,1,float>() || hasSplitForm<1,1,2,0,float>() ? &launch_split32_03_02 : nullptr;
+            else
+                return hasSplitForm<2,0,1,1,double>() || hasSplitForm<1,1,2,0,double>() ? &launch_split64_03_02 : nullptr;
+        case 303:
+            if (fp32)
+                return hasSplitForm<2,0,2,0,float>() || hasSplitForm<2,0,2,0,float>() ? &launch_split32_03_03 : nullptr;
+            else
+                return hasSplitForm<2,0,2,0,double>() || hasSplitForm<2,0,2,0,double>() ? &launch_split64_03_03 : nullptr;
+        case 400:
+            if (fp32)
+                return hasSplitForm<2,1,0,0,float>() || hasSplitForm<0,0,2,1,float>() ? &launch_split32_04_00 : nullptr;
+            else
+                return hasSplitForm<2,1,0,0,double>() || hasSplitForm<0,0,2,1,double>() ? &launch_split64_04_00 : nullptr;
+        case 401:
+            if (fp32)
+                return hasSplitForm<2,1,1,0,float>() || hasSplitForm<1,0,2,1,float>() ? &launch_split32_04_01 : nullptr;
+            else
+                return hasSplitForm<2,1,1,0,double>() || hasSplitForm<1,0,2,1,double>() ? &launch_split64_04_01 : nullptr;
+        case 402:
+            if (fp32)
+                return hasSplitForm<2,1,1,1,float>() || hasSplitForm<1,1,2,1,float>() ? &launch_split32_04_02 : nullptr;
+            else
+                return hasSplitForm<2,1,1,1,double>() || hasSplitForm<1,1,2,1,double>() ? &launch_split64_04_02 : nullptr;
+        case 403:
+            if (fp32)
+                return hasSplitForm<2,1,2,0,float>() || hasSplitForm<2,0,2,1,float>() ? &launch_split32_04_03 : nullptr;
+            else
+                return hasSplitForm<2,1,2,0,double>() || hasSplitForm<2,0,2,1,double>() ? &launch_split64_04_03 : nullptr;
+        case 404:
+            if (fp32)
+                return hasSplitForm<2,1,2,1,float>() || hasSplitForm<2,1,2,1,float>() ? &launch_split32_04_04 : nullptr;
+            else
+                return hasSplitForm<2,1,2,1,double>() || hasSplitForm<2,1,2,1,double>() ? &launch_split64_04_04 : nullptr;
+        case 500:
+            if (fp32)
+                return hasSplitForm<2,2,0,0,float>() || hasSplitForm<0,0,2,2,float>() ? &launch_split32_05_00 : nullptr;
+            else
+                return hasSplitForm<2,2,0,0,double>() || hasSplitForm<0,0,2,2,double>() ? &launch_split64_05_00 : nullptr;
+        case 501:
+            if (fp32)
+                return hasSplitForm<2,2,1,0,float>() || hasSplitForm<1,0,2,2,float>() ? &launch_split32_05_01 : nullptr;
+            else
+                return hasSplitForm<2,2,1,0,double>() || hasSplitForm<1,0,2,2,double>() ? &launch_split64_05_01 : nullptr;
+        case 502:
+            if (fp32)
+                return hasSplitForm<2,2,1,1,float>() || hasSplitForm<1,1,2,2,float>() ? &launch_split32_05_02 : nullptr;
+            else
+                return hasSplitForm<2,2,1,1,double>() || hasSplitForm<1,1,2,2,double>() ? &launch_split64_05_02 : nullptr;
+        case 503:
+            if (fp32)
+                return hasSplitForm<2,2,2,0,float>() || hasSplitForm<2,0,2,2,float>() ? &launch_split32_05_03 : nullptr;
+            else
+                return hasSplitForm<2,2,2,0,double>() || hasSplitForm<2,0,2,2,double>() ? &launch_split64_05_03 : nullptr;
+        case 600:
+            if (fp32)
+                return hasSplitForm<3,0,0,0,float>() || hasSplitForm<0,0,3,0,float>() ? &launch_split32_06_00 : nullptr;
+            else
+                return hasSplitForm<3,0,0,0,double>() || hasSplitForm<0,0,3,0,double>() ? &launch_split64_06_00 : nullptr;
+        case 601:
+            if (fp32)
+                return hasSplitForm<3,0,1,0,float>() || hasSplitForm<1,0,3,0,float>() ? &launch_split32_06_01 : nullptr;
+            else
+                return hasSplitForm<3,0,1,0,double>() || hasSplitForm<1,0,3,0,double>() ? &launch_split64_06_01 : nullptr;
+        case 602:
+            if (fp32)
+                return hasSplitForm<3,0,1,1,float>() || hasSplitForm<1,1,3,0,float>() ? &launch_split32_06_02 : nullptr;
+            else
+                return hasSplitForm<3,0,1,1,double>() || hasSplitForm<1,1,3,0,double>() ? &launch_split64_06_02 : nullptr;
+        case 603:
+            if (fp32)
+                return hasSplitForm<3,0,2,0,float>() || hasSplitForm<2,0,3,0,float>() ? &launch_split32_06_03 : nullptr;
+            else
+                return hasSplitForm<3,0,2,0,double>() || hasSplitForm<2,0,3,0,double>() ? &launch_split64_06_03 : nullptr;
+        case 604:
+            if (fp32)
+                return hasSplitForm<3,0,2,1,float>() || hasSplitForm<2,1,3,0,float>() ? &launch_split32_06_04 : nullptr;
+            else
+                return hasSplitForm<3,0,2,1,double>() || hasSplitForm<2,1,3,0,double>() ? &launch_split64_06_04 : nullptr;
+        case 606:
+            if (fp32)
+                return hasSplitForm<3,0,3,0,float>() || hasSplitForm<3,0,3,0,float>() ? &launch_split32_06_06 : nullptr;
+            else
+                return hasSplitForm<3,0,3,0,double>() || hasSplitForm<3,0,3,0,double>() ? &launch_split64_06_06 : nullptr;
+        case 700:
+            if (fp32)
+                return hasSplitForm<3,1,0,0,float>() || hasSplitForm<0,0,3,1,float>() ? &launch_split32_07_00 : nullptr;
+            else
+                return hasSplitForm<3,1,0,0,double>() || hasSplitForm<0,0,3,1,double>() ? &launch_split64_07_00 : nullptr;
+        case 701:
+            if (fp32)
+                return hasSplitForm<3,1,1,0,float>() || hasSplitForm<1,0,3,1,float>() ? &launch_split32_07_01 : nullptr;
+            else
+                return hasSplitForm<3,1,1,0,double>() || hasSplitForm<1,0,3,1,double>() ? &launch_split64_07_01 : nullptr;
+        case 702:
+            if (fp32)
+                return hasSplitForm<3,1,1,1,float>() || hasSplitForm<1,1,3,1,float>() ? &launch_split32_07_02 : nullptr;
+            else
+                return hasSplitForm<3,1,1,1,double>() || hasSplitForm<1,1,3,1,double>() ? &launch_split64_07_02 : nullptr;
+        case 703:
+            if (fp32)
+                return hasSplitForm<3,1,2,0,float>() || hasSplitForm<2,0,3,1,float>() ? &launch_split32_07_03 : nullptr;
+            else
+                return hasSplitForm<3,1,2,0,double>() || hasSplitForm<2,0,3,1,double>() ? &launch_split64_07_03 : nullptr;
+        case 800:
+            if (fp32)
+                return hasSplitForm<3,2,0,0,float>() || hasSplitForm<0,0,3,2,float>() ? &launch_split32_08_00 : nullptr;
+            else
+                return hasSplitForm<3,2,0,0,double>() || hasSplitForm<0,0,3,2,double>() ? &launch_split64_08_00 : nullptr;
+        case 801:
+            if (fp32)
+                return hasSplitForm<3,2,1,0,float>() || hasSplitForm<1,0,3,2,float>() ? &launch_split32_08_01 : nullptr;
+            else
+                return hasSplitForm<3,2,1,0,double>() || hasSplitForm<1,0,3,2,double>() ? &launch_split64_08_01 : nullptr;
+        case 900:
+            if (fp32)
+                return hasSplitForm<3,3,0,0,float>() || hasSplitForm<0,0,3,3,float>() ? &launch_split32_09_00 : nullptr;
+            else
+                return hasSplitForm<3,3,0,0,double>() || hasSplitForm<0,0,3,3,double>() ? &launch_split64_09_00 : nullptr;
+        default:
+            return nullptr;
+        }
+    }
+    bool splitFlipped(int bt, int kt, bool fp32)
+    {
+        switch (100 * bt + kt)
+        {
+        case 0:
+            if (fp32)
+                return !hasSplitForm<0,0,0,0,float>();
+            else
+                return !hasSplitForm<0,0,0,0,double>();
+        case 100:
+            if (fp32)
+                return !hasSplitForm<1,0,0,0,float>();
+            else
+                return !hasSplitForm<1,0,0,0,double>();
+        case 101:
+            if (fp32)
+                return !hasSplitForm<1,0,1,0,float>();
+            else
+                return !hasSplitForm<1,0,1,0,double>();
+        case 200:
+            if (fp32)
+                return !hasSplitForm<1,1,0,0,float>();
+            else
+                return !hasSplitForm<1,1,0,0,double>();
+        case 201:
+            if (fp32)
+                return !hasSplitForm<1,1,1,0,float>();
+            else
+                return !hasSplitForm<1,1,1,0,double>();
+        case 202:
+            if (fp32)
+                return !hasSplitForm<1,1,1,1,float>();
+            else
+                return !hasSplitForm<1,1,1,1,double>();
+        case 300:
+            if (fp32)
+                return !hasSplitForm<2,0,0,0,float>();
+            else
+                return !hasSplitForm<2,0,0,0,double>();
+        case 301:
+            if (fp32)
+                return !hasSplitForm<2,0,1,0,float>();
+            else
+                return !hasSplitForm<2,0,1,0,double>();
+        case 302:
+            if (fp32)
+                return !hasSplitForm<2,0,1,1,float>();
+            else
+                return !hasSplitForm<2,0,1,1,double>();
+        case 303:
+            if (fp32)
+                return !hasSplitForm<2,0,2,0,float>();
+            else
+                return !hasSplitForm<2,0,2,0,double>();
+        case 400:
+            if (fp32)
+                return !hasSplitForm<2,1,0,0,float>();
+            else
+                return !hasSplitForm<2,1,0,0,double>();
+        case 401:
+            if (fp32)
+                return !hasSplitForm<2,1,1,0,float>();
+            else
+                return !hasSplitForm<2,1,1,0,double>();
+        case 402:
+            if (fp32)
+                return !hasSplitForm<2,1,1,1,float>();
+            else
+                return !hasSplitForm<2,1,1,1,double>();
+        case 403:
+            if (fp32)
+                return !hasSplitForm<2,1,2,0,float>();
+            else
+                return !hasSplitForm<2,1,2,0,double>();
+        case 404:
+            if (fp32)
+                return !hasSplitForm<2,1,2,1,float>();
+            else
+                return !hasSplitForm<2,1,2,1,double>();
+        case 500:
+            if (fp32)
+                return !hasSplitForm<2,2,0,0,float>();
+            else
+                return !hasSplitForm<2,2,0,0,double>();
+        case 501:
+            if (fp32)
+                return !hasSplitForm<2,2,1,0,float>();
+            else
+                return !hasSplitForm<2,2,1,0,double>();
+        case 502:
+            if (fp32)
+                return !hasSplitForm<2,2,1,1,float>();
+            else
+                return !hasSplitForm<2,2,1,1,double>();
+        case 503:
+            if (fp32)
+                return !hasSplitForm<2,2,2,0,float>();
+            else
+                return !hasSplitForm<2,2,2,0,double>();
+        case 600:
+            if (fp32)
+                return !hasSplitForm<3,0,0,0,float>();
+            else
+                return !hasSplitForm<3,0,0,0,double>();
+        case 601:
+            if (fp32)
+                return !hasSplitForm<3,0,1,0,float>();
+            else
+                return !hasSplitForm<3,0,1,0,double>();
+        case 602:
+            if (fp32)
+                return !hasSplitForm<3,0,1,1,float>();
+            else
+                return !hasSplitForm<3,0,1,1,double>();
+        case 603:
+            if (fp32)
+                return !hasSplitForm<3,0,2,0,float>();
+            else
+                return !hasSplitForm<3,0,2,0,double>();
+        case 604:
+            if (fp32)
+                return !hasSplitForm<3,0,2,1,float>();
+            else
+                return !hasSplitForm<3,0,2,1,double>();
+        case 606:
+            if (fp32)
+                return !hasSplitForm<3,0,3,0,float>();
+            else
+                return !hasSplitForm<3,0,3,0,double>();
+        case 700:
+            if (fp32)
+                return !hasSplitForm<3,1,0,0,float>();
+            else
+                return !hasSplitForm<3,1,0,0,double>();
+        case 701:
+            if (fp32)
+                return !hasSplitForm<3,1,1,0,float>();
+            else
+                return !hasSplitForm<3,1,1,0,double>();
+        case 702:
+            if (fp32)
+                return !hasSplitForm<3,1,1,1,float>();
+            else
+                return !hasSplitForm<3,1,1,1,double>();
+        case 703:
+            if (fp32)
+                return !hasSplitForm<3,1,2,0,float>();
+            else
+                return !hasSplitForm<3,1,2,0,double>();
+        case 800:
+            if (fp32)
+                return !hasSplitForm<3,2,0,0,float>();
+            else
+                return !hasSplitForm<3,2,0,0,double>();
+        case 801:
+            if (fp32)
+                return !hasSplitForm<3,2,1,0,float>();
+            else
+                return !hasSplitForm<3,2,1,0,double>();
+        case 900:
+            if (fp32)
+                return !hasSplitForm<3,3,0,0,float>();
+            else
+                return !hasSplitForm<3,3,0,0,double>();
+        default:
+            return false;
+        }
+    }
     LaunchFn lookupFwd64(int bt, int kt, int shape)
     {
         if (bt < 0 || bt >= 12 || kt < 0 || kt > bt)

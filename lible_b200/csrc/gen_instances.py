@@ -18,6 +18,17 @@ def kinds():
     yield "d1", "launchD1<{la},{lb},{lc},{ld}>", len(PAIR_TYPES)
 
 
+# split forms (eri_split_kernel.cuh): total angular momentum up to 6 over the l <= 3 pair types, in the
+# orientation that takes the register path
+SPLIT_MAX_L = 6
+
+
+def split_classes():
+    n = FP32_MAX_TYPE + 1
+    return [(bt, kt) for bt in range(n) for kt in range(bt + 1)
+            if sum(PAIR_TYPES[bt]) + sum(PAIR_TYPES[kt]) <= SPLIT_MAX_L]
+
+
 # classes per generated file: small groups keep every nvcc invocation short, so a rebuild spreads
 # over all cores instead of waiting on the files of the largest bra types
 GROUP = {"fwd64": 2, "fwd32": 2, "d1": 3}
@@ -29,7 +40,7 @@ def main():
     os.makedirs(out, exist_ok=True)
     written = []
     table = ['// Generated by gen_instances.py: lookup of class kernels.',
-             '#include "../eri_launch_fwd.cuh"', '', 'namespace lible_b200', '{']
+             '#include "../eri_launch_fwd.cuh"', '#include "../eri_split_kernel.cuh"', '', 'namespace lible_b200', '{']
     for kind, tmpl, ntypes in kinds():
         launcher = "launchD1" if kind == "d1" else "launchFwd"
         T = {"fwd64": ",double", "fwd32": ",float", "d1": ""}[kind]
@@ -99,6 +110,45 @@ def main():
                          ", ".join(f"k_{kind}f_{bt:02d}" for bt in range(ntypes)) + '};')
         table.append(f'    static const LaunchFn *const k_{kind}[{ntypes}] = {{' +
                      ", ".join(f"k_{kind}_{bt:02d}" for bt in range(ntypes)) + '};')
+    for T, tag in (("double", "64"), ("float", "32")):
+        classes = split_classes()
+        for g in range(0, len(classes), 3):
+            part = classes[g:g + 3]
+            body = ['// Generated by gen_instances.py: split forms of ' +
+                    ", ".join("(%d,%d|%d,%d)" % (PAIR_TYPES[bt] + PAIR_TYPES[kt]) for bt, kt in part) + '.',
+                    '#include "../eri_launch_fwd.cuh"', '#include "../eri_split_kernel.cuh"', '',
+                    'namespace lible_b200', '{']
+            for bt, kt in part:
+                d = "%d,%d,%d,%d,%s" % (PAIR_TYPES[bt] + PAIR_TYPES[kt] + (T,))
+                f = "%d,%d,%d,%d,%s" % (PAIR_TYPES[kt] + PAIR_TYPES[bt] + (T,))
+                body += [f'    cudaError_t launch_split{tag}_{bt:02d}_{kt:02d}(const QuartetArgs &a, cudaStream_t s, int n)',
+                         '    {', f'        if constexpr (hasSplitForm<{d}>())',
+                         f'            return launchSplit<{d}>(a, s, n);', '        else',
+                         f'            return launchSplit<{f}>(a, s, n);', '    }']
+            body += ['}', '']
+            name = f"inst_split{tag}_{g // 3:03d}.cu"
+            path = os.path.join(out, name)
+            text = "\n".join(body)
+            if not os.path.exists(path) or open(path).read() != text:
+                with open(path, "w") as fh:
+                    fh.write(text)
+            written.append(name)
+        table += [f'    cudaError_t launch_split{tag}_{bt:02d}_{kt:02d}(const QuartetArgs &, cudaStream_t, int);'
+                  for bt, kt in classes]
+    for fn, ret, null in (("lookupSplit", "LaunchFn", "nullptr"), ("splitFlipped", "bool", "false")):
+        table += [f'    {ret} {fn}(int bt, int kt, bool fp32)', '    {', '        switch (100 * bt + kt)', '        {']
+        for bt, kt in split_classes():
+            d = lambda T: "%d,%d,%d,%d,%s" % (PAIR_TYPES[bt] + PAIR_TYPES[kt] + (T,))
+            f = lambda T: "%d,%d,%d,%d,%s" % (PAIR_TYPES[kt] + PAIR_TYPES[bt] + (T,))
+            table.append(f'        case {100 * bt + kt}:')
+            for cond, T, tag in (("if (fp32)", "float", "32"), ("else", "double", "64")):
+                table.append(f'            {cond}')
+                if fn == "lookupSplit":
+                    table.append(f'                return hasSplitForm<{d(T)}>() || hasSplitForm<{f(T)}>() ? '
+                                 f'&launch_split{tag}_{bt:02d}_{kt:02d} : nullptr;')
+                else:
+                    table.append(f'                return !hasSplitForm<{d(T)}>();')
+        table += ['        default:', f'            return {null};', '        }', '    }']
     for kind, _, ntypes in kinds():
         fn = {"fwd64": "lookupFwd64", "fwd32": "lookupFwd32", "d1": "lookupD1"}[kind]
         if kind == "d1":

@@ -97,6 +97,9 @@ namespace lible_b200
         a.mode = kStore;
         a.out = out_dev;
         LaunchFn fn = lookupFwd64(swap ? tk : tb, swap ? tb : tk);
+        if (splitStore(bra, ket, n) && !splitFlipped(swap ? tk : tb, swap ? tb : tk, false))
+            if (const LaunchFn sf = lookupSplit(swap ? tk : tb, swap ? tb : tk, false))
+                fn = sf;
         if (!fn)
             throw EngineError(kStatusUnsupported, "quartet class not instantiated");
         cudaCheck(fn(a, stream_, num_sms_), "eri kernel");
