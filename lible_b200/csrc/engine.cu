@@ -1257,18 +1257,18 @@ namespace lible_b200
     // it holds the cost of `unit` tasks of the most expensive run (one full worker step of the
     // heaviest quartets) or `max_tasks` tasks, whichever comes first; with the heaviest runs first
     // in the task order and chunks claimed dynamically, the last chunks to finish are cheap ones.
-    static std::vector<unsigned long long> costChunks(const std::vector<unsigned long long> &n,
-                                                      const std::vector<double> &c, int unit, int max_tasks)
+    // Runs [lo, hi) are cut, and the boundaries appended to `ch`, whose last entry is where they begin.
+    static void costChunks(const std::vector<unsigned long long> &n, const std::vector<double> &c, size_t lo, size_t hi,
+                           int unit, int max_tasks, std::vector<unsigned long long> &ch)
     {
         double cmax = 0;
-        for (size_t i = 0; i < n.size(); i++)
+        for (size_t i = lo; i < hi; i++)
             if (n[i])
                 cmax = std::max(cmax, c[i]);
         const double C = (double)std::max(unit, 1) * cmax;
-        std::vector<unsigned long long> ch(1, 0);
-        unsigned long long pos = 0, cnt = 0;
+        unsigned long long pos = ch.back(), cnt = 0;
         double acc = 0;
-        for (size_t i = 0; i < n.size(); i++)
+        for (size_t i = lo; i < hi; i++)
         {
             unsigned long long left = n[i];
             while (left > 0)
@@ -1296,7 +1296,6 @@ namespace lible_b200
         }
         if (ch.back() != pos)
             ch.push_back(pos);
-        return ch;
     }
 
     // Surviving quartets of one class pair, kept iff Q_bra Q_ket >= thr (and, with `triangle`, only
@@ -1529,14 +1528,10 @@ namespace lible_b200
         const auto &runs = fp32 ? cp.run32 : cp.run64;
         const size_t lead = cp.split && lookupSplit(tb, tk, fp32) ? splitRuns(runs, cp.cost, unit, num_sms_) : 0;
         // the split launch's chunks first (runs come heaviest first), one to four tasks each
-        auto ch = costChunks({runs.begin(), runs.begin() + lead}, {cp.cost.begin(), cp.cost.begin() + lead}, 1,
-                             mult > 1 ? 4 : 1);
+        std::vector<unsigned long long> ch(1, 0);
+        costChunks(runs, cp.cost, 0, lead, 1, mult > 1 ? 4 : 1, ch);
         (fp32 ? cp.n_split32 : cp.n_split64) = (long long)ch.size() - 1;
-        const auto rest =
-            costChunks({runs.begin() + lead, runs.end()}, {cp.cost.begin() + lead, cp.cost.end()}, unit, mult * unit);
-        const unsigned long long base = ch.back();
-        for (size_t i = 1; i < rest.size(); i++)
-            ch.push_back(base + rest[i]);
+        costChunks(runs, cp.cost, lead, runs.size(), unit, mult * unit, ch);
         (fp32 ? cp.n_chunks32 : cp.n_chunks64) = (long long)ch.size() - 1;
         dev = devUpload(ch, stream_);
     }
@@ -1580,6 +1575,12 @@ namespace lible_b200
         return plans_.emplace(key, std::move(plan)).first->second;
     }
 
+    // A build whose launches do not fill the device (about 5 ms of FP64 work).
+    bool Engine::smallPlan(const JKPlan &plan)
+    {
+        return plan.flops64 + 0.5 * plan.flops32 < 2e10;
+    }
+
     // Longest-processing-time assignment of the class pairs (already in decreasing cost) to the
     // stream branches of the fork/join launch sequence, so the tail of one class kernel overlaps
     // the next ones.
@@ -1589,7 +1590,7 @@ namespace lible_b200
         // a small build's launches each leave most of the device idle and last as long as their longest
         // quartet, so they run side by side on all streams; launches that fill the device gain nothing
         // from more than four
-        const int nb = plan.flops64 + 0.5 * plan.flops32 < 2e10 ? kBranches : 4;
+        const int nb = smallPlan(plan) ? kBranches : 4;
         for (auto &cp : plan.pairs)
         {
             int b = 0;
@@ -2101,6 +2102,40 @@ namespace lible_b200
     // ------------------------------------------------------------------------------------------
     // J/K energy gradient (adjoint of the J/K build): dE/dR over all unique quartets.
 
+    // Work-queue chunks of a gradient launch: one quartet per worker step (block or warp forms) or 32 / gt
+    // (register form), up to 8 steps a chunk, fewer where the launch has too few tasks to give every
+    // resident worker (16 per SM) a chunk.
+    void Engine::ensureChunksD1(JKClassPair &cp, const DevPairClass &B, const DevPairClass &K)
+    {
+        if (cp.chunksD1 || cp.t64 <= 0)
+            return;
+        const int gt = d1WarpClass(B.la, B.lb, K.la, K.lb) ? 0 : d1RegisterGroup(B.la, B.lb, K.la, K.lb);
+        const int unit = gt ? 32 / gt : 1;
+        const int mult = (int)std::min<long long>(8, std::max<long long>(1, cp.t64 / (16LL * num_sms_ * unit)));
+        std::vector<unsigned long long> ch(1, 0);
+        costChunks(cp.run64, cp.cost, 0, cp.run64.size(), unit, mult * unit, ch);
+        cp.n_chunksD1 = (long long)ch.size() - 1;
+        cp.chunksD1 = devUpload(ch, stream_);
+    }
+
+    // Fork of the stream branches: launches on branch_[b], b < nb, follow everything on stream_.
+    void Engine::forkBranches(int nb)
+    {
+        cudaCheck(cudaEventRecord(fork_, stream_), "fork");
+        for (int b = 0; b < nb; b++)
+            cudaCheck(cudaStreamWaitEvent(branch_[b], fork_, 0), "fork");
+    }
+
+    // Join: stream_ waits for the branches.
+    void Engine::joinBranches(int nb)
+    {
+        for (int b = 0; b < nb; b++)
+        {
+            cudaCheck(cudaEventRecord(join_[b], branch_[b]), "join");
+            cudaCheck(cudaStreamWaitEvent(stream_, join_[b], 0), "join");
+        }
+    }
+
     // The quartets are those of the FP64 J/K plan with the same Schwarz threshold, so the gradient
     // is the exact derivative of the energy lible_gpu_jk_energy_forward computes with that threshold.
     void Engine::jkGradient(const double *D_dev, double *grad_dev, double schwarz)
@@ -2112,20 +2147,18 @@ namespace lible_b200
         cudaCheck(cudaMemsetAsync(grad_dev, 0, 3 * n_atoms_ * sizeof(double), stream_), "memset");
         cudaCheck(cudaMemsetAsync(plan.counters, 0, 2 * plan.pairs.size() * sizeof(unsigned long long), stream_),
                   "memset");
+        // chunks first: their uploads must precede the fork
+        for (auto &cp : plan.pairs)
+            ensureChunksD1(cp, cs.dev[cp.cb], cs.dev[cp.ck]);
+        // Small plans overlap their launches, each of which leaves most of the device idle; the launches of
+        // large ones fill it and run one after another (on four streams the (H2O)_8 cc-pVTZ gradient took
+        // 434 ms, against 317 ms of kernels)
+        const int nb = smallPlan(plan) ? kBranches : 0;
+        forkBranches(nb);
         for (size_t ip = 0; ip < plan.pairs.size(); ip++)
         {
             auto &cp = plan.pairs[ip];
             const auto &B = cs.dev[cp.cb], &K = cs.dev[cp.ck];
-            if (!cp.chunksD1 && cp.t64 > 0)
-            {
-                // one quartet per block at a time: chunks of the heaviest quartet up to 8 tasks; the
-                // register classes take 32 quartets per warp step
-                const int gt = d1RegisterGroup(B.la, B.lb, K.la, K.lb);
-                const int unit = gt ? 32 / gt : 1;
-                auto ch = costChunks(cp.run64, cp.cost, unit, 8 * unit);
-                cp.n_chunksD1 = (long long)ch.size() - 1;
-                cp.chunksD1 = devUpload(ch, stream_);
-            }
             QuartetArgs a{};
             a.bra = view(B);
             a.ket = view(K);
@@ -2152,8 +2185,10 @@ namespace lible_b200
             a.chunks = cp.chunksD1;
             a.n_chunks = cp.n_chunksD1;
             a.counter = plan.counters + 2 * ip;
-            cudaCheck(lookupD1(pairType(B.la, B.lb), pairType(K.la, K.lb))(a, stream_, num_sms_), "grad kernel");
+            cudaCheck(lookupD1(pairType(B.la, B.lb), pairType(K.la, K.lb))(a, nb ? branch_[cp.branch] : stream_, num_sms_),
+                      "grad kernel");
         }
+        joinBranches(nb);
         cudaCheck(cudaStreamSynchronize(stream_), "grad");
     }
 
@@ -2295,22 +2330,22 @@ namespace lible_b200
         for (JKPlan *plan : {&p3, &p2})
         {
             const bool two = plan == &p2;
+            for (auto &cp : plan->pairs)
+                ensureChunksD1(cp, (two || cp.swap ? xs : ms).dev[cp.cb], (!two && cp.swap ? ms : xs).dev[cp.ck]);
             cudaCheck(cudaMemsetAsync(plan->counters, 0, 2 * plan->pairs.size() * sizeof(unsigned long long), stream_),
                       "memset");
+        }
+        forkBranches(kBranches);
+        int branch = 0;  // launches dealt out in turn: each leaves part of the device idle at its end
+        for (JKPlan *plan : {&p3, &p2})
+        {
+            const bool two = plan == &p2;
             for (size_t ip = 0; ip < plan->pairs.size(); ip++)
             {
                 auto &cp = plan->pairs[ip];
                 const ClassSet &bs = two ? xs : (cp.swap ? xs : ms);
                 const ClassSet &ks = two ? xs : (cp.swap ? ms : xs);
                 const auto &B = bs.dev[cp.cb], &K = ks.dev[cp.ck];
-                if (!cp.chunksD1 && cp.t64 > 0)
-                {
-                    const int gt = d1RegisterGroup(B.la, B.lb, K.la, K.lb);
-                    const int unit = gt ? 32 / gt : 1;
-                    auto ch = costChunks(cp.run64, cp.cost, unit, 8 * unit);
-                    cp.n_chunksD1 = (long long)ch.size() - 1;
-                    cp.chunksD1 = devUpload(ch, stream_);
-                }
                 QuartetArgs a{};
                 a.bra = view(B);
                 a.ket = view(K);
@@ -2340,9 +2375,11 @@ namespace lible_b200
                 a.chunks = cp.chunksD1;
                 a.n_chunks = cp.n_chunksD1;
                 a.counter = plan->counters + 2 * ip;
-                cudaCheck(lookupD1(pairType(B.la, B.lb), pairType(K.la, K.lb))(a, stream_, num_sms_), "ri grad");
+                cudaCheck(lookupD1(pairType(B.la, B.lb), pairType(K.la, K.lb))(a, branch_[branch++ % kBranches], num_sms_),
+                          "ri grad");
             }
         }
+        joinBranches(kBranches);
         cudaCheck(cudaStreamSynchronize(stream_), "ri grad");
         checkStatus();
     }

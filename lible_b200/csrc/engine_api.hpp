@@ -295,6 +295,10 @@ namespace lible_b200
         void rebuildChunks(JKClassPair &cp, bool fp32, int mult);
         // Whether a store launch of n quartets of two classes splits every quartet over a warp.
         bool splitStore(const DevPairClass &bra, const DevPairClass &ket, long long n) const;
+        void ensureChunksD1(JKClassPair &cp, const DevPairClass &B, const DevPairClass &K);
+        void forkBranches(int nb);
+        void joinBranches(int nb);
+        static bool smallPlan(const JKPlan &plan);
         void assignBranches(JKPlan &plan);
         struct LaunchTimer;
         QuartetArgs jkArgs(const JKPlan &plan, size_t ip, bool fp32, bool mixed, const double *D, double *J, double *K);

@@ -469,7 +469,8 @@ namespace lible_b200
     //   tc_x  = sum GE  . (-(c/q) dR/dP_x E_cd^T + R E1_cd,x^T),
     // and A_x += (a/p) t1_x + t13_x, B_x += (b/p) t1_x - t13_x, C_x += tc_x (D by invariance).
     template <int LA, int LB, int LC, int LD>
-    __device__ __forceinline__ void quartetD1Reg(const QuartetArgs &a, uint32_t ib, uint32_t ik, int c0, double *g)
+    __device__ __forceinline__ void quartetD1Reg(const QuartetArgs &a, uint32_t ib, uint32_t ik, int c0,
+                                                 const double *btab, double *g)
     {
         using C = Cls<LA, LB, LC, LD>;
         constexpr int L1 = C::L + 1;
@@ -560,7 +561,7 @@ namespace lible_b200
                 const double X = P.y - Q.y, Y = P.z - Q.z, Z = P.w - Q.w;
                 const double fac = 34.986836655249725 * rs * P.ip * Q.ip;
                 double F[L1 + 1];
-                boysF<L1, false>(alpha * (X * X + Y * Y + Z * Z), a.boys + L1 * kBoysTerms * kBoysPitch, F);
+                boysF<L1, true>(alpha * (X * X + Y * Y + Z * Z), btab, F);
 #pragma unroll
                 for (int k = 0; k <= L1; k++)
                     F[k] *= fac;
@@ -634,6 +635,8 @@ namespace lible_b200
     __global__ void __launch_bounds__(128) eriD1RegKernel(QuartetArgs a)
     {
         extern __shared__ __align__(16) double sg[];
+        __shared__ double btab[kBoysTerms * kBoysPitch];  // the order-(L + 1) Boys table
+        stageBoys(a.boys, LA + LB + LC + LD + 1, btab);
         for (int e = threadIdx.x; e < 3 * a.n_atoms; e += blockDim.x)
             sg[e] = 0.0;
         __syncthreads();
@@ -663,7 +666,7 @@ namespace lible_b200
                     decodeCursor(a, t, my, ib, ik);
                     active = inWindow(a, ib, ik, 0, false);
                     if (active)
-                        quartetD1Reg<LA, LB, LC, LD>(a, ib, ik, member * CW, g);
+                        quartetD1Reg<LA, LB, LC, LD>(a, ib, ik, member * CW, btab, g);
                 }
                 if (!a.list)
                     cur = advanceMajor(a, base + QPW < end ? base + QPW : end - 1, cur);

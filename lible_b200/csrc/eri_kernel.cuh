@@ -296,6 +296,75 @@ namespace lible_b200
         groupSync(G);
     }
 
+    // Warp form of the McMurchie-Davidson recursion, for kernels that keep one quartet per warp.  Entry e
+    // of every level comes from the level above by one rule, R_e = x R_i1 + c R_i2 (x the entry's axis
+    // of (X, Y, Z)), so a block keeps the rules of its entries in shared memory (buildWarpRules): packed
+    // i1 | i2 << 10 | axis << 20, and c.  L + 1 warp barriers and about a third of the instructions of the
+    // closed form above, which pays where a barrier costs a whole block.
+    __device__ __forceinline__ void buildWarpRules(int n_entries, uint32_t *rule, double *coef)
+    {
+        for (int e = threadIdx.x; e < n_entries; e += blockDim.x)
+        {
+            int t, u, v;
+            hermTuv(e, t, u, v);
+            const int axis = t > 0 ? 0 : u > 0 ? 1 : 2, k = axis == 0 ? t : axis == 1 ? u : v;
+            uint32_t i1 = 0, i2 = 0;
+            if (e > 0)
+            {
+                i1 = (uint32_t)hermIndex(t - (axis == 0), u - (axis == 1), v - (axis == 2));
+                i2 = k > 1 ? (uint32_t)hermIndex(t - 2 * (axis == 0), u - 2 * (axis == 1), v - 2 * (axis == 2)) : i1;
+            }
+            rule[e] = i1 | i2 << 10 | (uint32_t)axis << 20;
+            coef[e] = k > 1 ? k - 1 : 0;
+        }
+    }
+    // R_tuv, t + u + v <= L, from F_n (all lanes alike) into one of the two buffers of nherm(L) doubles at
+    // `buf`; returns it.  `xyz`: three doubles of the warp's shared memory.  The first barrier also ends
+    // the warp's earlier reads of the buffers.
+    template <int L>
+    __device__ __forceinline__ const double *warpHermiteR(const double (&F)[L + 1], double fac, double m2a, double X,
+                                                          double Y, double Z, double *buf, double *xyz,
+                                                          const uint32_t *rule, const double *coef, int lane)
+    {
+        double gf[L + 1], pw = fac;
+#pragma unroll
+        for (int n = 0; n <= L; n++)
+        {
+            gf[n] = F[n] * pw;
+            pw *= m2a;
+        }
+        double *cur = buf + (L & 1) * nherm(L), *nxt = buf + (1 - (L & 1)) * nherm(L);
+        __syncwarp();
+        if (lane < 3)
+            xyz[lane] = lane == 0 ? X : lane == 1 ? Y : Z;
+        if (lane == 0)
+            cur[0] = gf[L];
+        __syncwarp();
+#pragma unroll
+        for (int n = L - 1; n >= 0; n--)
+        {
+            const int cnt = nherm(L - n);
+#pragma unroll
+            for (int k = 0; k < (cnt + 31) / 32; k++)
+            {
+                const int e = lane + 32 * k;
+                if (e < cnt)
+                {
+                    const uint32_t ru = rule[e];
+                    double r = xyz[ru >> 20] * cur[ru & 1023] + coef[e] * cur[(ru >> 10) & 1023];
+                    if (k == 0 && lane == 0)
+                        r = gf[n];
+                    nxt[e] = r;
+                }
+            }
+            __syncwarp();
+            double *tmp = cur;
+            cur = nxt;
+            nxt = tmp;
+        }
+        return cur;
+    }
+
     template <typename T>
     __device__ __forceinline__ const T *braE(const PairView &v);
     template <>

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "eri_d1_kernel.cuh"
+#include "eri_d1_warp.cuh"
 #include "eri_launch.cuh"
 
 #include <algorithm>
@@ -14,12 +15,15 @@ namespace lible_b200
         using S = ShapeD1<LA, LB, LC, LD>;
         if (a.n_tasks <= 0)
             return cudaSuccess;
-        if constexpr (d1RegisterClass(LA, LB, LC, LD))
+        if constexpr (d1WarpClass(LA, LB, LC, LD))
+            if (a.mode == kD1Grad || a.mode == kD1GradRI)
+                return launchD1Warp<LA, LB, LC, LD>(a, s, num_sms);
+        if constexpr (d1RegisterClass(LA, LB, LC, LD) && !d1WarpClass(LA, LB, LC, LD))
         {
             // J/K gradient of the smallest classes: one quartet per thread, the block's gradient in
-            // shared memory (up to 2,048 atoms)
+            // shared memory (up to 1,877 atoms)
             const size_t sg = sizeof(double) * 3 * (size_t)std::max(a.n_atoms, 1);
-            if ((a.mode == kD1Grad || a.mode == kD1GradRI) && a.n_atoms > 0 && sg <= 48 * 1024)
+            if ((a.mode == kD1Grad || a.mode == kD1GradRI) && a.n_atoms > 0 && sg <= 44 * 1024)
             {
                 auto rk = eriD1RegKernel<LA, LB, LC, LD>;
                 int occ = 0;
@@ -32,7 +36,7 @@ namespace lible_b200
                 return cudaGetLastError();
             }
         }
-        if constexpr (ShapeD1M<LA, LB, LC, LD>::USE)
+        if constexpr (ShapeD1M<LA, LB, LC, LD>::USE && !d1WarpClass(LA, LB, LC, LD))
         {
             // gradient epilogues of the larger classes: both contractions on the DMMA pipe
             if (a.mode == kD1Grad || a.mode == kD1GradRI)

@@ -101,6 +101,21 @@ namespace lible_b200
         return d1RegisterGroup(la, lb, lc, ld) > 0;
     }
 
+    // Derivative classes whose gradient contraction runs one warp per quartet (eriD1WarpKernel): bras of
+    // at least 35 Hermite functions, whose rows fill the warp once or twice, or the 20 of (dp), and of
+    // (fs) under kets of 9 functions or more; kets thin enough that a lane's rows of the four
+    // Gamma-weighted bra matrices (4 x S_cd values each) stay within 72 doubles.  Kernel times of the
+    // (H2O)_8 cc-pVTZ gradient against the block, tensor-pipe or register form that served the class:
+    // (fd|ps) 26.1 -> 3.5 ms, (dd|ps) 22.6 -> 6.3, (fp|ps) 20.6 -> 6.2, (dd|ds) 14.5 -> 5.7,
+    // (dd|pp) 9.9 -> 4.9, (dp|pp) 16.3 -> 10.7, (dp|dp) 13.6 -> 9.0, (dp|ps) 17.3 -> 16.4; the whole
+    // gradient 437 -> 280 ms.  (fs) bras under thinner kets stay on the register form ((fs|ps) 5.4 ms).
+    LB_HD constexpr bool d1WarpClass(int la, int lb, int lc, int ld)
+    {
+        const int hab = nherm(la + lb), scd = nsph(lc) * nsph(ld);
+        return (hab >= 35 || (hab >= 20 && (lb > 0 || scd >= 9))) && 4 * scd * ((hab + 31) / 32) <= 72 &&
+               la + lb + lc + ld + 1 <= 10;
+    }
+
     // Hermite expansion coefficients of a primitive pair along one axis, McMurchie-Davidson
     // recurrences (Helgaker, Jorgensen, Olsen, Molecular Electronic-Structure Theory, 9.5.6-9.5.7).
     // E[i][j][t] is stored at E[(i * (lb + 1) + j) * (la + lb + 1) + t].  `one_o_2p` = 1/(2p),
