@@ -3,11 +3,20 @@
 
 #include "eri_kernel.cuh"
 #include "eri_launch.cuh"
+#include "eri_warp_kernel.cuh"
 
 #include <algorithm>
 
 namespace lible_b200
 {
+    // FP64 classes whose default is the warp form (shape variant 1 and the other orientation keep the
+    // register or block kernels, which the autotuner times against it).
+    template <int LA, int LB, int LC, int LD, typename T, int SV>
+    constexpr bool usesWarpForm()
+    {
+        return sizeof(T) == 8 && SV == 0 && warpClass(LA, LB, LC, LD);
+    }
+
     // Quartets a worker processes side by side: QPW per warp on the register path, one per block on
     // the group path.  Work-queue chunks are cut so that each holds at least one unit of the most
     // expensive quartets.
@@ -15,7 +24,7 @@ namespace lible_b200
     constexpr int workUnit()
     {
         using S = Shape<LA, LB, LC, LD, T, SV>;
-        return S::W == 0 ? S::QPW : 1;
+        return S::W == 0 && !usesWarpForm<LA, LB, LC, LD, T, SV>() ? S::QPW : 1;
     }
 
     template <int LA, int LB, int LC, int LD, typename T, int SV = 0>
@@ -24,6 +33,10 @@ namespace lible_b200
         using S = Shape<LA, LB, LC, LD, T, SV>;
         if (a.n_tasks <= 0)
             return cudaSuccess;
+        if constexpr (usesWarpForm<LA, LB, LC, LD, T, SV>())
+            return launchWarp<LA, LB, LC, LD>(a, s, num_sms);
+        else
+        {
         auto kern = eriKernelFor<LA, LB, LC, LD, T, SV>();
         long long grid;
         if (a.chunks)
@@ -72,6 +85,7 @@ namespace lible_b200
         }
         kern<<<(unsigned)grid, S::block, S::smem, s>>>(a);
         return cudaGetLastError();
+        }
     }
 
 }
