@@ -914,7 +914,7 @@ int lible_gpu_jk_energy_backward(lible_gpu_ctx *ctx, const double *D, const libl
         if (!D || !grad)
             throw EngineError(kStatusInvalid, "null D/grad");
         const size_t n = e.nao();
-        DevArray d(D, n * n, true, e.stream());
+        DevArray d(D, n * n, true, e.stream(), &e, 0);
         DevArray g(grad, 3 * (size_t)e.nAtoms(), false, e.stream());
         e.jkGradient(d.ptr, g.ptr, toOpts(opts).schwarz);
         g.copyOut();
@@ -969,8 +969,8 @@ int lible_gpu_rij(lible_gpu_ctx *ctx, const double *D, double schwarz_threshold,
         if (!D || !J)
             throw EngineError(kStatusInvalid, "null D/J");
         const size_t n = e.nao(), na = e.naux();
-        DevArray d(D, n * n, true, e.stream());
-        DevArray j(J, n * n, false, e.stream());
+        DevArray d(D, n * n, true, e.stream(), &e, 0);
+        DevArray j(J, n * n, false, e.stream(), &e, 1);
         DevBuf<double> rhs_b(na);
         double *rhs = rhs_b.p;
         // the tensor (naux * nao (nao + 1) / 2 doubles) is built by the first call when it takes at
@@ -1036,7 +1036,8 @@ int lible_gpu_one_electron(lible_gpu_ctx *ctx, const double *charges, int n_char
         if (charges && n_charges < 0)
             throw EngineError(kStatusInvalid, "negative n_charges");
         const size_t n = e.nao();
-        DevArray s(S, n * n, false, e.stream()), t(T, n * n, false, e.stream()), v(V, n * n, false, e.stream());
+        DevArray s(S, n * n, false, e.stream(), &e, 0), t(T, n * n, false, e.stream(), &e, 1),
+            v(V, n * n, false, e.stream(), &e, 2);
         e.oneElectron(charges, charges ? n_charges : 0, charges == nullptr, s.ptr, t.ptr, v.ptr);
         e.sync();
         s.copyOut();
@@ -1175,7 +1176,7 @@ int lible_gpu_rij_grad(lible_gpu_ctx *ctx, const double *D, double schwarz_thres
         if (!D || !grad)
             throw EngineError(kStatusInvalid, "null D/grad");
         const size_t n = e.nao(), na = e.naux();
-        DevArray d(D, n * n, true, e.stream());
+        DevArray d(D, n * n, true, e.stream(), &e, 0);
         DevArray g(grad, (size_t)e.nAtoms() * 3, false, e.stream());
         DevBuf<double> rhs(na);
         e.riContract(d.ptr, nullptr, rhs.p, nullptr, schwarz_threshold);
@@ -1206,7 +1207,7 @@ int lible_gpu_rik(lible_gpu_ctx *ctx, const double *D, const double *C, long lon
         if (C && n_occ < 0)
             throw EngineError(kStatusInvalid, "negative n_occ");
         const size_t n = e.nao();
-        DevArray k(K, n * n, false, e.stream());
+        DevArray k(K, n * n, false, e.stream(), &e, 1);
         cudaCheck(cudaMemsetAsync(k.ptr, 0, n * n * sizeof(double), e.stream()), "memset");
         const MetricFactor &mf = ctx->metricFactor(e);
         BlasHandle &bh = ctx->blasHandle(e);
@@ -1242,12 +1243,12 @@ int lible_gpu_rik(lible_gpu_ctx *ctx, const double *D, const double *C, long lon
         };
         if (C)
         {
-            DevArray c(C, n * (size_t)std::max<long long>(n_occ, 1), true, e.stream());
+            DevArray c(C, n * (size_t)std::max<long long>(n_occ, 1), true, e.stream(), &e, 2);
             exchange(c.ptr, n_occ, 1.0);
         }
         else
         {
-            DevArray d(D, n * n, true, e.stream());
+            DevArray d(D, n * n, true, e.stream(), &e, 0);
             DevBuf<double> cp, cm;
             splitDensity(e, d.ptr, (long long)n, cp, n_pos, cm, n_neg);
             exchange(cp.p, n_pos, 1.0);

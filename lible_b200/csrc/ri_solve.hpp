@@ -90,6 +90,10 @@ namespace lible_b200
         // of method 0 (a positive definite metric), so that every solve is one symmetric
         // matrix-vector product; the shifted and eigen methods keep their solves
         mutable DevBuf<double> inv;
+        // method 0: the metric itself (both triangles), for the residual of the refinement step, and
+        // the solve's solution vector
+        DevBuf<double> mat;
+        mutable DevBuf<double> x;
         // solver and cuBLAS handles of the solves, created once
         mutable std::unique_ptr<SolverHandle> solver;
         mutable std::unique_ptr<BlasHandle> blas;
