@@ -256,6 +256,22 @@ namespace lible_b200
         cudaCheck(cudaGetLastError(), "mirror");
     }
 
+    // The symmetric metric M (n x n) laid beside its Cholesky factor: the strict upper triangle (column-major)
+    // into the half of `fac` that the factor does not use, the diagonal into `diag`.
+    __global__ void keepMetricKernel(const double *__restrict__ M, int n, double *__restrict__ fac,
+                                     double *__restrict__ diag)
+    {
+        const long long nn = (long long)n * n;
+        for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn; e += (long long)gridDim.x * blockDim.x)
+        {
+            const int i = (int)(e % n), j = (int)(e / n);
+            if (i < j)
+                fac[e] = M[e];
+            else if (i == j)
+                diag[i] = M[e];
+        }
+    }
+
     void factorMetric(Engine &e, MetricFactor &mf)
     {
         const size_t na = e.naux();
@@ -317,8 +333,11 @@ namespace lible_b200
             mf.method = shift > 0 ? 2 : 0;
             if (mf.method == 0)
             {
-                std::swap(mf.mat.p, copy.p);
-                std::swap(mf.mat.n, copy.n);
+                // the metric beside its factor, for the refinement of the solves
+                mf.diag.reset(na);
+                keepMetricKernel<<<gridFor((long long)(na * na)), 256, 0, s>>>(copy.p, (int)na, metric, mf.diag.p);
+                cudaCheck(cudaGetLastError(), "metric copy");
+                cudaCheck(cudaStreamSynchronize(s), "metric copy");
             }
             mf.lo = lo;
             mf.hi = hi;
@@ -366,31 +385,60 @@ namespace lible_b200
         mf.dropped = dropped;
     }
 
-    // r_i -= sum_j M_ij x_j, one warp per row of the full metric (rows streamed once, x from L2).  It replaces
-    // the two triangular products with the Cholesky factor, which ran at 0.15 TB/s: 0.69 ms of an RI-J
-    // call with 3,616 auxiliary functions.
-    __global__ void __launch_bounds__(256) metricResidualKernel(const double *__restrict__ M, const double *__restrict__ x,
-                                                                int n, double *__restrict__ r)
+    // r_i -= sum_j M_ij x_j with the metric kept beside its factor (keepMetricKernel): M_ij, i < j, in column
+    // j of U, the diagonal in d.  A block of 32 warps takes 32 rows: warp k the dot product of
+    // column r0 + k above its diagonal (M_ji, j < i, contiguous), then the lanes take the 32 rows and the
+    // warps the columns to their right (M_ij, j > i, 256 bytes a column), summed over the warps in shared memory.
+    // Every element is read twice, n^2 doubles in all, as by one pass over a full copy of the metric,
+    // which would cost every context naux^2 doubles, also one that only builds exchange.
+    // Bound by the loads in flight of n / 32 blocks: 24.6 us at 3,616 functions (4.3 TB/s), 26 us by rows
+    // of a full copy; two triangular products with the factor took 0.69 ms.
+    __global__ void __launch_bounds__(1024) metricResidualKernel(const double *__restrict__ U, const double *__restrict__ d,
+                                                                 const double *__restrict__ x, int n, double *__restrict__ r)
     {
-        const int row = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
-        if (row >= n)
-            return;
-        const double *m = M + (size_t)row * n;
+        __shared__ double part[32][33];
+        const int r0 = (int)blockIdx.x * 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = r0 + warp;
         double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        int j = lane;
-        for (; j + 96 < n; j += 128)
+        if (row < n)
         {
-            s0 = fma(__ldg(m + j), __ldg(x + j), s0);
-            s1 = fma(__ldg(m + j + 32), __ldg(x + j + 32), s1);
-            s2 = fma(__ldg(m + j + 64), __ldg(x + j + 64), s2);
-            s3 = fma(__ldg(m + j + 96), __ldg(x + j + 96), s3);
+            const double *m = U + (size_t)row * n;
+            int j = lane;
+            for (; j + 96 < row; j += 128)
+            {
+                s0 = fma(__ldg(m + j), __ldg(x + j), s0);
+                s1 = fma(__ldg(m + j + 32), __ldg(x + j + 32), s1);
+                s2 = fma(__ldg(m + j + 64), __ldg(x + j + 64), s2);
+                s3 = fma(__ldg(m + j + 96), __ldg(x + j + 96), s3);
+            }
+            for (; j < row; j += 32)
+                s0 = fma(__ldg(m + j), __ldg(x + j), s0);
+            if (lane == 0)
+                s1 = fma(__ldg(d + row), __ldg(x + row), s1);
         }
-        for (; j < n; j += 32)
-            s0 = fma(__ldg(m + j), __ldg(x + j), s0);
-        double s = (s0 + s1) + (s2 + s3);
+        const int mine = r0 + lane;
+        double u0 = 0.0, u1 = 0.0, u2 = 0.0, u3 = 0.0;
+        if (mine < n)
+        {
+            const double *m = U + mine;
+            int j = r0 + 1 + warp;  // the first column of a warp may lie left of a lane's row; the later ones do not
+            if (j < n && j > mine)
+                u0 = __ldg(m + (size_t)j * n) * __ldg(x + j);
+            for (j += 32; j + 96 < n; j += 128)
+            {
+                u0 = fma(__ldg(m + (size_t)j * n), __ldg(x + j), u0);
+                u1 = fma(__ldg(m + (size_t)(j + 32) * n), __ldg(x + j + 32), u1);
+                u2 = fma(__ldg(m + (size_t)(j + 64) * n), __ldg(x + j + 64), u2);
+                u3 = fma(__ldg(m + (size_t)(j + 96) * n), __ldg(x + j + 96), u3);
+            }
+            for (; j < n; j += 32)
+                u0 = fma(__ldg(m + (size_t)j * n), __ldg(x + j), u0);
+        }
+        part[warp][lane] = (u0 + u1) + (u2 + u3);
+        __syncthreads();
+        double s = ((s0 + s1) + (s2 + s3)) + part[lane][warp];
         for (int o = 16; o > 0; o >>= 1)
             s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0)
+        if (row < n && lane == 0)
             r[row] -= s;
     }
 
@@ -446,7 +494,7 @@ namespace lible_b200
             // x0 = M^{-1} b
             blasCheck(cublasDsymv(h, CUBLAS_FILL_MODE_LOWER, na, &one, mf.inv.p, na, rhs, 1, &zero, x, 1), "symv");
             // r = b - M x0 (in place of b), then x = x0 + M^{-1} r
-            metricResidualKernel<<<(na + 7) / 8, 256, 0, s>>>(mf.mat.p, x, na, rhs);
+            metricResidualKernel<<<(na + 31) / 32, 1024, 0, s>>>(mf.fac.p, mf.diag.p, x, na, rhs);
             cudaCheck(cudaGetLastError(), "metric residual");
             blasCheck(cublasDsymv(h, CUBLAS_FILL_MODE_LOWER, na, &one, mf.inv.p, na, rhs, 1, &one, x, 1), "symv");
             cudaCheck(cudaMemcpyAsync(rhs, x, mf.naux * sizeof(double), cudaMemcpyDeviceToDevice, s), "copy");

@@ -90,9 +90,10 @@ namespace lible_b200
         // of method 0 (a positive definite metric), so that every solve is one symmetric
         // matrix-vector product; the shifted and eigen methods keep their solves
         mutable DevBuf<double> inv;
-        // method 0: the metric itself (both triangles), for the residual of the refinement step, and
-        // the solve's solution vector
-        DevBuf<double> mat;
+        // method 0 keeps the metric itself for the residual of the refinement step, its strict upper
+        // triangle in the half of `fac` that L does not use and its diagonal here; `x` is the solve's
+        // solution vector
+        DevBuf<double> diag;
         mutable DevBuf<double> x;
         // solver and cuBLAS handles of the solves, created once
         mutable std::unique_ptr<SolverHandle> solver;
