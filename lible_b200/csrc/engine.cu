@@ -1967,7 +1967,6 @@ namespace lible_b200
         for (size_t ip = 0; ip < plan.pairs.size(); ip++)
         {
             JKClassPair &cp = plan.pairs[ip];
-            const auto &B = cs.dev[cp.cb];
             for (int fp32 = 0; fp32 < (mixed ? 2 : 1); fp32++)
             {
                 const long long n = fp32 ? cp.t32 : cp.t64;
@@ -1980,30 +1979,28 @@ namespace lible_b200
                         shapes[n_shapes++] = s2;
                 float best = 1e30f;
                 int best_gd = 1, best_cm = 8, best_shape = 0;
+                bool choice = false;  // some candidate has an ordinary launch
                 for (int si = 0; si < n_shapes; si++)
                 for (int cm : mults)
                 {
-                    const int shape = shapes[si];
-                    LaunchFn fn = fp32 ? lookupFwd32(cp.tb, cp.tk, shape) : lookupFwd64(cp.tb, cp.tk, shape);
-                    if (!fn)
-                        throw EngineError(kStatusUnsupported, "quartet class not instantiated");
-                    (fp32 ? cp.shape32 : cp.shape64) = shape;
+                    (fp32 ? cp.shape32 : cp.shape64) = shapes[si];
                     rebuildChunks(cp, fp32 == 1, cm);  // the work unit depends on the shape
                     for (int gd : grid_divs)
                     {
-                        QuartetArgs a = jkArgs(plan, ip, fp32 == 1, mixed, D, J, K);
-                        if (a.n_chunks <= 0)
-                            continue;  // every quartet in the split launch
-                        a.grid_div = gd;
-                        if (shape == 2)
-                            flipOrientation(a, B.EtP);
-                        // a second timing only for short launches, where one sample is noisy
+                        (fp32 ? cp.grid_div32 : cp.grid_div64) = gd;
+                        choice |= (fp32 ? cp.n_chunks32 > cp.n_split32 : cp.n_chunks64 > cp.n_split64);
+                        // the split launch too: which quartets go to it depends on the shape, so only the
+                        // sum compares equal work.  A second timing only for short launches, where one
+                        // sample is noisy
                         float t_min = 1e30f;
                         for (int rep = 0; rep < 2 && (rep == 0 || t_min < 2.0f); rep++)
                         {
-                            cudaCheck(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), stream_), "memset");
+                            cudaCheck(cudaMemsetAsync(plan.counters, 0, 4 * plan.pairs.size() * sizeof(unsigned long long),
+                                                      stream_),
+                                      "memset");
                             cudaCheck(cudaEventRecord(e0, stream_), "event");
-                            cudaCheck(fn(a, stream_, num_sms_), "autotune kernel");
+                            launchSplitJK(plan, ip, fp32 == 1, mixed, D, J, K, stream_);
+                            launchClassJK(plan, ip, fp32 == 1, mixed, D, J, K, stream_);
                             cudaCheck(cudaEventRecord(e1, stream_), "event");
                             cudaCheck(cudaEventSynchronize(e1), "event");
                             float ms = 0;
@@ -2015,13 +2012,23 @@ namespace lible_b200
                             best = t_min;
                             best_gd = gd;
                             best_cm = cm;
-                            best_shape = shape;
+                            best_shape = shapes[si];
                         }
                     }
+                }
+                if (!choice)
+                {
+                    // every quartet in the split launch, which has nothing to choose: the defaults, and no
+                    // entry that another molecule's ordinary launch of this size would take for a choice
+                    best_gd = 1;
+                    best_cm = 8;
+                    best_shape = 0;
                 }
                 (fp32 ? cp.shape32 : cp.shape64) = best_shape;
                 rebuildChunks(cp, fp32 == 1, best_cm);
                 (fp32 ? cp.grid_div32 : cp.grid_div64) = best_gd;
+                if (!choice)
+                    continue;
                 const auto &Bh = cs.host[cp.cb], &Kh = cs.host[cp.ck];
                 char line[320];
                 snprintf(line, sizeof(line), "%s|%d %d %d %d|%d|%d|%d %d %d\n", gpu_name_.c_str(), Bh.la, Bh.lb, Kh.la,
