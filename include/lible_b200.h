@@ -175,7 +175,8 @@ int lible_gpu_batch_layout(lible_gpu_ctx *ctx, int *n_mol, long long *nao, long 
  * ((cd|ab) for (ab|cd), where that orientation takes the register path), resident blocks per SM
  * (all or half) and work-queue chunks of 2, 8 or 32 work units.  J and K are overwritten with
  * meaningless values.  When cache_path is non-empty the choices are appended to that text file;
- * lible_gpu_set_tune_cache(ctx, path) makes later plans start from a cache.  summary (may be NULL)
+ * lible_gpu_set_tune_cache(ctx, path) makes later plans start from a cache; entries written for an older
+ * set of kernels are not used.  summary (may be NULL)
  * receives one line per class pair; a class pair whose quartets are all heavily contracted runs them one
  * per warp, which leaves nothing to choose, and gets no line and no entry. */
 int lible_gpu_jk_autotune(lible_gpu_ctx *ctx, const double *D, double *J, double *K, const lible_gpu_jk_opts *opts,

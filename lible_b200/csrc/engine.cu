@@ -1887,16 +1887,22 @@ namespace lible_b200
     // Autotuning of the class-pair launches.  The tunable "tile" of a persistent class kernel is
     // its occupancy (resident blocks per SM divided by grid_div) and the granularity of its work
     // queue (chunks of at most chunk_mult work units); every candidate is timed on the caller's
-    // buffers with CUDA events and the fastest is kept.  Results are keyed by GPU name, quartet
-    // class and the size bucket floor(log2(tasks)), and appended to a plain-text cache:
-    //     <gpu>|<la> <lb> <lc> <ld>|<fp32>|<bucket>|<grid_div> <chunk_mult>
+    // buffers with CUDA events and the fastest is kept.  Results are keyed by GPU name, kernel set,
+    // quartet class and the size bucket floor(log2(tasks)), and appended to a plain-text cache:
+    //     <gpu> k<set>|<la> <lb> <lc> <ld>|<fp32>|<bucket>|<grid_div> <chunk_mult> <shape>
+    // The kernel set is raised when a shape of a J/K class gets another kernel, so that choices made against
+    // the old one are not taken over (set 2: the warp and split forms; lines before it name no set).
 
-    static int sizeBucket(long long n)
+    constexpr int kKernelSet = 2;
+
+    static std::string tuneKey(const std::string &gpu, int la, int lb, int lc, int ld, int fp32, long long tasks)
     {
-        int b = 0;
-        while ((1LL << (b + 1)) <= n)
-            b++;
-        return b;
+        int bucket = 0;
+        while ((1LL << (bucket + 1)) <= tasks)
+            bucket++;
+        char key[256];
+        snprintf(key, sizeof(key), "%s k%d|%d %d %d %d|%d|%d", gpu.c_str(), kKernelSet, la, lb, lc, ld, fp32, bucket);
+        return key;
     }
 
     void Engine::applyTuneCache(JKPlan &plan)
@@ -1932,10 +1938,7 @@ namespace lible_b200
                 if (n == 0)
                     continue;
                 const auto &B = cs.host[cp.cb], &K = cs.host[cp.ck];
-                char key[256];
-                snprintf(key, sizeof(key), "%s|%d %d %d %d|%d|%d", gpu_name_.c_str(), B.la, B.lb, K.la, K.lb, fp32,
-                         sizeBucket(n));
-                auto it = entries.find(key);
+                auto it = entries.find(tuneKey(gpu_name_, B.la, B.lb, K.la, K.lb, fp32, n));
                 if (it == entries.end())
                     continue;
                 const Choice &ch = it->second;
@@ -2030,11 +2033,11 @@ namespace lible_b200
                 if (!choice)
                     continue;
                 const auto &Bh = cs.host[cp.cb], &Kh = cs.host[cp.ck];
-                char line[320];
-                snprintf(line, sizeof(line), "%s|%d %d %d %d|%d|%d|%d %d %d\n", gpu_name_.c_str(), Bh.la, Bh.lb, Kh.la,
-                         Kh.lb, fp32, sizeBucket(n), best_gd, best_cm, best_shape);
+                const std::string line = tuneKey(gpu_name_, Bh.la, Bh.lb, Kh.la, Kh.lb, fp32, n) + "|" +
+                                         std::to_string(best_gd) + " " + std::to_string(best_cm) + " " +
+                                         std::to_string(best_shape) + "\n";
                 if (out)
-                    fputs(line, out);
+                    fputs(line.c_str(), out);
                 char info[200];
                 snprintf(info, sizeof(info), "(%d%d|%d%d) %s tasks=%lld shape=%d grid_div=%d chunk_mult=%d %.3f ms\n",
                          Bh.la, Bh.lb, Kh.la, Kh.lb, fp32 ? "fp32" : "fp64", n, best_shape, best_gd, best_cm, best);

@@ -4,6 +4,7 @@ import re
 
 import numpy as np
 import pytest
+import torch
 
 from lible_b200 import ints as L
 from lible_b200.workloads import random_density, water_cluster
@@ -43,3 +44,21 @@ def test_a_class_without_an_ordinary_launch_leaves_no_entry(tmp_path):
     assert cache.read_text() == ""
     Jt, Kt, _ = L.jk(s, D, schwarz=0.0)
     assert np.abs(Jt - J).max() <= 1e-12 and np.abs(Kt - K).max() <= 1e-12
+
+
+def test_choices_of_older_kernels_are_not_taken_over(tmp_path):
+    """A cache whose lines name the GPU alone, as before the warp and split forms, with the other orientation
+    for every class."""
+    Z, xyz, rng = water_cluster(1, seed=52)
+    s = L.Structure("cc-pvtz", Z, xyz, units="bohr")
+    D = random_density(s.nao, 5, rng)
+    cache = tmp_path / "tune.txt"
+    L.jk_autotune(s, D, cache=str(cache))
+    gpu = torch.cuda.get_device_name(0)
+    lines = cache.read_text().splitlines()
+    assert lines and all(x.startswith(gpu) for x in lines)
+    old = [f"{gpu}|{x.split('|', 1)[1].rsplit(' ', 1)[0]} 2" for x in lines]
+    cache.write_text("\n".join(old) + "\n")
+    s2 = L.Structure("cc-pvtz", Z, xyz, units="bohr")
+    L.set_tune_cache(s2, str(cache))
+    assert {r["shape"] for r in L.jk_profile(s2, D)} == {0}
