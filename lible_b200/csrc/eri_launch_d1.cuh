@@ -21,11 +21,18 @@ namespace lible_b200
         if constexpr (d1RegisterClass(LA, LB, LC, LD) && !d1WarpClass(LA, LB, LC, LD))
         {
             // J/K gradient of the smallest classes: one quartet per thread, the block's gradient in
-            // shared memory (up to 1,877 atoms)
+            // shared memory (up to 2,048 atoms)
             const size_t sg = sizeof(double) * 3 * (size_t)std::max(a.n_atoms, 1);
-            if ((a.mode == kD1Grad || a.mode == kD1GradRI) && a.n_atoms > 0 && sg <= 44 * 1024)
+            if ((a.mode == kD1Grad || a.mode == kD1GradRI) && a.n_atoms > 0 && sg <= 48 * 1024)
             {
                 auto rk = eriD1RegKernel<LA, LB, LC, LD>;
+                // beside it the kernel's Boys table: together above the 48 KB a block gets unasked
+                if (sg + sizeof(double) * kBoysTerms * kBoysPitch > 48 * 1024)
+                {
+                    const cudaError_t e = cudaFuncSetAttribute(rk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sg);
+                    if (e != cudaSuccess)
+                        return e;
+                }
                 int occ = 0;
                 cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rk, 128, sg);
                 if (e != cudaSuccess)
