@@ -1519,9 +1519,14 @@ namespace lible_b200
             return;
         // bra / ket classes of the launch: the bra set is the auxiliary one for swapped RI pairs
         const int tb = cp.tb, tk = cp.tk;
-        const int unit = unitFwd(tb, tk, fp32, fp32 ? cp.shape32 : cp.shape64);
+        int unit = unitFwd(tb, tk, fp32, fp32 ? cp.shape32 : cp.shape64);
         if (unit == 0)
             return;
+        int la, lb, lc, ld;
+        pairTypeMomenta(tb, la, lb);
+        pairTypeMomenta(tk, lc, ld);
+        if (warpWhileShort(la, lb, lc, ld) && n < shortLaunch(num_sms_))
+            unit = 1;  // the warp form
         // a launch with few tasks is cut finer, down to one worker step a chunk, so that its chunks reach
         // every resident worker (16 warps, or as many blocks, per SM)
         mult = (int)std::min<long long>(mult, std::max<long long>(1, n / (16LL * num_sms_ * unit)));

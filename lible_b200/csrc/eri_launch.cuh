@@ -17,6 +17,13 @@ namespace lible_b200
             return la * (la + 1) / 2 + lb;
         return la == 4 ? 10 : 11;
     }
+    inline void pairTypeMomenta(int type, int &la, int &lb)
+    {
+        la = type < 10 ? 0 : type - 6;
+        while (type < 10 && (la + 1) * (la + 2) / 2 <= type)
+            la++;
+        lb = type < 10 ? type - la * (la + 1) / 2 : 0;
+    }
 
     // Implemented by the generated instantiation files.
     // `shape` selects the tile-shape variant of the forward class kernels (0 default, 1 the

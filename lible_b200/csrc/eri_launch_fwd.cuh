@@ -24,19 +24,15 @@ namespace lible_b200
     constexpr int workUnit()
     {
         using S = Shape<LA, LB, LC, LD, T, SV>;
-        return S::W == 0 && !usesWarpForm<LA, LB, LC, LD, T, SV>() ? S::QPW : 1;
+        constexpr bool warp = usesWarpForm<LA, LB, LC, LD, T, SV>() && !warpWhileShort(LA, LB, LC, LD);
+        return S::W == 0 && !warp ? S::QPW : 1;
     }
 
-    template <int LA, int LB, int LC, int LD, typename T, int SV = 0>
-    cudaError_t launchFwd(const QuartetArgs &a, cudaStream_t s, int num_sms)
+    // Register or group path of a class.
+    template <int LA, int LB, int LC, int LD, typename T, int SV>
+    cudaError_t launchPath(const QuartetArgs &a, cudaStream_t s, int num_sms)
     {
         using S = Shape<LA, LB, LC, LD, T, SV>;
-        if (a.n_tasks <= 0)
-            return cudaSuccess;
-        if constexpr (usesWarpForm<LA, LB, LC, LD, T, SV>())
-            return launchWarp<LA, LB, LC, LD>(a, s, num_sms);
-        else
-        {
         auto kern = eriKernelFor<LA, LB, LC, LD, T, SV>();
         long long grid;
         if (a.chunks)
@@ -85,7 +81,20 @@ namespace lible_b200
         }
         kern<<<(unsigned)grid, S::block, S::smem, s>>>(a);
         return cudaGetLastError();
-        }
+    }
+
+    template <int LA, int LB, int LC, int LD, typename T, int SV = 0>
+    cudaError_t launchFwd(const QuartetArgs &a, cudaStream_t s, int num_sms)
+    {
+        if (a.n_tasks <= 0)
+            return cudaSuccess;
+        if constexpr (!usesWarpForm<LA, LB, LC, LD, T, SV>())
+            return launchPath<LA, LB, LC, LD, T, SV>(a, s, num_sms);
+        else if constexpr (!warpWhileShort(LA, LB, LC, LD))
+            return launchWarp<LA, LB, LC, LD>(a, s, num_sms);
+        else
+            return a.n_tasks < (a.chunks ? 1 : 2) * shortLaunch(num_sms) ? launchWarp<LA, LB, LC, LD>(a, s, num_sms)
+                                                                         : launchPath<LA, LB, LC, LD, T, SV>(a, s, num_sms);
     }
 
 }

@@ -18,7 +18,10 @@ namespace lible_b200
     // of one function with at least 84.  Measured on the (H2O)_8 cc-pVTZ J/K build against the register or
     // block kernel that served the class: (fd|ps) 7.24 -> 2.10 ms, (dd|pp) 4.83 -> 1.67, (fd|ds) 4.35 -> 1.37,
     // (dd|ps) 5.04 -> 3.26, (dd|ds) 4.13 -> 2.18, (fp|pp) 3.46 -> 1.67, (ff|ss) 1.73 -> 0.30; one function
-    // is too thin for the smaller bras ((dd|ss) 1.40 -> 2.10 ms, (fp|ss) 2.18 -> 2.14).
+    // is too thin for the smaller bras ((dd|ss) 1.40 -> 2.10 ms, (fp|ss) 2.18 -> 2.14).  Of the classes with
+    // an auxiliary shell, the RI contractions of (H2O)_12 cc-pVTZ with def2-qzvp-rifit: (hs|ps) 1.64 -> 0.49 ms,
+    // (hs|ds) 0.87 -> 0.34, (hs|pp) 0.84 -> 0.26, (gs|fs) 1.34 -> 0.46, (fd|fs) 1.12 -> 0.37, (ff|ss) 0.36 -> 0.11,
+    // (gs|pp) 0.95 -> 0.89; (gs|ps) and (gs|ds) only while short (warpWhileShort).
     constexpr bool warpClass(int la, int lb, int lc, int ld)
     {
         const int scd = nsph(lc) * nsph(ld);

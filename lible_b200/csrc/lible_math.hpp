@@ -116,6 +116,22 @@ namespace lible_b200
                la + lb + lc + ld + 1 <= 10;
     }
 
+    // Classes of the warp form (eriWarpKernel) that take it only in short launches, else their register kernel:
+    // (gs|ps) and (gs|ds).  A bra of 9 functions fills 9 lanes of the second contraction and its 35
+    // Hermite functions two rows of 32, so the warp form costs more a quartet, but a short launch waits
+    // for its longest chain.  Short is fewer than four quartets per warp slot (16 a SM) for a work queue,
+    // eight for a list, which comes in no order.  Measured, warp / register form in us: RI contractions of
+    // cc-pVTZ waters with def2-universal-jkfit, (gs|ps) 73 / 110 at 4,480 quartets, 89 / 104 at 8,750, 97 / 74
+    // at 15,120, 183 / 91 at 35,840; (gs|ds) 56 / 66 at 5,000, 80 / 70 at 8,640, 133 / 92 at 20,480;
+    // (H2O)_32 cc-pVDZ 2178 / 867 and 573 / 387.  Lists, (gs|ps) 68 / 138 at 9,472, 112 / 134 at 20,000,
+    // 178 / 144 at 40,000; (gs|ds) 69 / 109, 125 / 113, 211 / 172.
+    LB_HD constexpr bool warpWhileShort(int la, int lb, int lc, int ld)
+    {
+        const int scd = nsph(lc) * nsph(ld);
+        return nsph(la) * nsph(lb) < 11 && nherm(la + lb) >= 35 && scd >= 3 && scd <= 5;
+    }
+    LB_HD constexpr long long shortLaunch(int num_sms) { return 4LL * 16 * num_sms; }
+
     // Hermite expansion coefficients of a primitive pair along one axis, McMurchie-Davidson
     // recurrences (Helgaker, Jorgensen, Olsen, Molecular Electronic-Structure Theory, 9.5.6-9.5.7).
     // E[i][j][t] is stored at E[(i * (lb + 1) + j) * (la + lb + 1) + t].  `one_o_2p` = 1/(2p),
