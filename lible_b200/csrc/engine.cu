@@ -1580,10 +1580,10 @@ namespace lible_b200
         return plans_.emplace(key, std::move(plan)).first->second;
     }
 
-    // A build whose launches do not fill the device (about 5 ms of FP64 work).
-    bool Engine::smallPlan(const JKPlan &plan)
+    // A build whose launches do not fill the device, judged by its operations.
+    bool Engine::smallPlan(const JKPlan &plan, double limit)
     {
-        return plan.flops64 + 0.5 * plan.flops32 < 2e10;
+        return plan.flops64 + 0.5 * plan.flops32 < limit;
     }
 
     // Longest-processing-time assignment of the class pairs (already in decreasing cost) to the
@@ -1594,8 +1594,9 @@ namespace lible_b200
         double load[kBranches] = {};
         // a small build's launches each leave most of the device idle and last as long as their longest
         // quartet, so they run side by side on all streams; launches that fill the device gain nothing
-        // from more than four
-        const int nb = smallPlan(plan) ? kBranches : 4;
+        // from more than four.  Measured, 4 against 16 streams: (H2O)_8 cc-pVDZ (1.8e10 operations) 3.49 / 3.53 ms,
+        // (H2O)_10 (2.2e10) 4.53 / 4.24, (H2O)_12 (3.9e10) 7.28 / 7.32, (H2O)_4 cc-pVTZ (4.2e10) 10.85 / 10.78
+        const int nb = smallPlan(plan, 2e10) ? kBranches : 4;
         for (auto &cp : plan.pairs)
         {
             int b = 0;
@@ -2166,9 +2167,11 @@ namespace lible_b200
         for (auto &cp : plan.pairs)
             ensureChunksD1(cp, cs.dev[cp.cb], cs.dev[cp.ck]);
         // Small plans overlap their launches, each of which leaves most of the device idle; the launches of
-        // large ones fill it and run one after another (on four streams the (H2O)_8 cc-pVTZ gradient took
-        // 434 ms, against 317 ms of kernels)
-        const int nb = smallPlan(plan) ? kBranches : 0;
+        // large ones run in order.  Measured, in order against 16 streams: (H2O)_8 cc-pVDZ (1.8e10 operations)
+        // 19.8 / 13.7 ms, (H2O)_10 (2.2e10) 21.6 / 16.7, (H2O)_12 (3.9e10) 33.2 / 30.4, (H2O)_4 cc-pVTZ (4.2e10)
+        // 43.9 / 38.5, (H2O)_14 def2-SVP (4.4e10) 43.6 / 44.1, (H2O)_5 cc-pVTZ (7.6e10) 68.4 / 70.4, (H2O)_6 (1.4e11)
+        // 117.7 / 129.8, (H2O)_16 cc-pVDZ (1.1e11) 86.2 / 86.3
+        const int nb = smallPlan(plan, 4.3e10) ? kBranches : 0;
         forkBranches(nb);
         for (size_t ip = 0; ip < plan.pairs.size(); ip++)
         {
@@ -2350,8 +2353,11 @@ namespace lible_b200
             cudaCheck(cudaMemsetAsync(plan->counters, 0, 2 * plan->pairs.size() * sizeof(unsigned long long), stream_),
                       "memset");
         }
+        // Launches dealt out in turn to all branches, whatever the size: each leaves part of the device idle at
+        // its end.  Measured with def2-universal-jkfit, in order against 16 streams: (H2O)_1 cc-pVDZ 3.90 / 1.75 ms,
+        // (H2O)_8 5.99 / 4.07, (H2O)_16 15.8 / 14.4, (H2O)_32 65.5 / 64.9, (H2O)_4 cc-pVTZ 7.74 / 4.90
         forkBranches(kBranches);
-        int branch = 0;  // launches dealt out in turn: each leaves part of the device idle at its end
+        int branch = 0;
         for (JKPlan *plan : {&p3, &p2})
         {
             const bool two = plan == &p2;

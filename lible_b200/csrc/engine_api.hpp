@@ -298,7 +298,7 @@ namespace lible_b200
         void ensureChunksD1(JKClassPair &cp, const DevPairClass &B, const DevPairClass &K);
         void forkBranches(int nb);
         void joinBranches(int nb);
-        static bool smallPlan(const JKPlan &plan);
+        static bool smallPlan(const JKPlan &plan, double limit);
         void assignBranches(JKPlan &plan);
         struct LaunchTimer;
         QuartetArgs jkArgs(const JKPlan &plan, size_t ip, bool fp32, bool mixed, const double *D, double *J, double *K);
