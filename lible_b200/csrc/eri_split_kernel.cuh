@@ -33,7 +33,7 @@ namespace lible_b200
         static constexpr size_t smem = off_boys + S::boys_bytes;
     };
 
-    // Store, J/K and RI epilogues as the class kernels; tasks from the chunk queue, or one per warp
+    // J/K and (FP64) store epilogues as the class kernels; tasks from the chunk queue, or one per warp
     // without one.
     template <int LA, int LB, int LC, int LD, typename T>
     __global__ void __launch_bounds__(128) eriSplitKernel(QuartetArgs a)
@@ -98,17 +98,18 @@ namespace lible_b200
             const int32_t *bi = a.bra.info + 8 * ib;
             const int32_t *ki = a.ket.info + 8 * ik;
             auto val = [&](int e) { return vw[e]; };
-            if (a.mode == kStore)
+            bool store = false;
+            if constexpr (sizeof(T) == 8)
+                store = a.mode == kStore;
+            if (store)
                 for (int e = lane; e < blk; e += 32)
                 {
                     const int m = e / C::SCD, kt = e % C::SCD;
                     a.out[(size_t)t * blk + storeIndex<C::SA, C::SB, C::SC, C::SD>(a.flags, m / C::SB, m % C::SB,
                                                                                    kt / C::SD, kt % C::SD)] = vw[e];
                 }
-            else if (a.mode == kJK)
-                digestJK<C::SA, C::SB, C::SC, C::SD, false>(a, quartetWeight(a, ib, ik), braFields(bi), ki, val, lane, 32);
             else
-                digestRI<C::SA, C::SB, C::SC, C::SD, false>(a, bi, ki, val, lane, 32);
+                digestJK<C::SA, C::SB, C::SC, C::SD, false>(a, quartetWeight(a, ib, ik), braFields(bi), ki, val, lane, 32);
             __syncwarp();
         };
         if (a.chunks)
