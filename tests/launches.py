@@ -8,7 +8,7 @@ from torch.profiler import ProfilerActivity, profile
 def launched(call):
     """{kernel without its namespace, return type and arguments, e.g. eriSplitKernel<0,0,0,0,double>: launches}."""
     torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
         call()
         torch.cuda.synchronize()
     names = {}
