@@ -1312,7 +1312,9 @@ namespace lible_b200
     // total angular momentum is at least 8.  Measured per class on (H2O)_8 cc-pVTZ, the FP32
     // register or group kernels of those classes plus the FP64 launch of their large quartets took
     // longer than the DMMA kernel running all of their quartets ((fd|dp) 5.3 against 3.6 ms, (fp|dd)
-    // 3.5 against 2.0 ms, (fd|fp) 2.5 against 1.4 ms).
+    // 3.5 against 2.0 ms, (fd|fp) 2.5 against 1.4 ms).  Not among them are the classes that the FP64 warp
+    // form serves, of which several are slower in FP32 too ((fd|fs) 32.8 against 9.4 ns a quartet, (ff|pp)
+    // 42.5 / 14.6, (dd|pp) 7.8 / 5.2); the autotuner finds another FP32 shape for some.
     static bool fp32InFp64(int la, int lb, int lc, int ld)
     {
         const int sab = nsph(la) * nsph(lb), scd = nsph(lc) * nsph(ld);
@@ -1470,14 +1472,14 @@ namespace lible_b200
     // the thread groups of a warp.  A quartet's primitive pairs are otherwise one thread group's serial
     // chain (64 x 64 pairs of two contracted core pairs: about 1.6 ms of (ss|ss) on an otherwise idle
     // device), so a launch cannot end before the chain of its heaviest quartet.  Split are the
-    // quartets with at least as many pairs as every resident group (16 warps per SM) gets when the
-    // launch is spread evenly, and at least 32 (8 when every quartet can have a warp of its own): with
-    // fewer the reduction and the digestion by one quartet cost more than the chain.  Measured: (ss|ss)
-    // of (H2O)_16 cc-pVDZ 2.64 -> 1.56 ms, of one water 1.61 -> 0.10 ms; with the finer chunks and 16
-    // streams of small plans the whole J/K of one water went from 2.38 to 0.25 ms, of (H2O)_5 def2-SVP
-    // from 1.38 to 0.76 ms.  Splitting from half or a quarter of the even share on slows the classes that
-    // fill the device anyway ((dp|ss) of (H2O)_16 0.89 -> 0.99 ms), from 14 pairs on the (H2O)_5 build
-    // (1.21 ms).
+    // quartets whose cost (primitive pairs + 4, as everywhere in the plans) is at least what every resident
+    // group (16 warps per SM) gets when the launch is spread evenly, and at least 32, that is 28 pairs (8,
+    // that is 4 pairs, when every quartet can have a warp of its own): with fewer the reduction and the
+    // digestion by one quartet cost more than the chain.  Measured: (ss|ss) of (H2O)_16 cc-pVDZ
+    // 2.64 -> 1.56 ms, of one water 1.61 -> 0.10 ms; with the finer chunks and 16 streams of small plans the
+    // whole J/K of one water went from 2.38 to 0.25 ms, of (H2O)_5 def2-SVP from 1.38 to 0.76 ms.  Splitting
+    // from half or a quarter of the even share on slows the classes that fill the device anyway ((dp|ss) of
+    // (H2O)_16 0.89 -> 0.99 ms), from 14 pairs on the (H2O)_5 build (1.21 ms).
     static size_t splitRuns(const std::vector<unsigned long long> &n, const std::vector<double> &c, int unit, int num_sms)
     {
         double total = 0;
@@ -1497,7 +1499,10 @@ namespace lible_b200
 
     // Store launches take explicit lists whose contraction lengths the host does not look at: every
     // quartet is split when the class averages at least 4 primitive pairs per quartet and the list
-    // would not give each warp slot of the device (16 per SM) 8 quartets.
+    // would not give each warp slot of the device (16 per SM) 8 quartets.  Both lines are cautious: over the
+    // classes of 6-31+G, cc-pVDZ, def2-SVP and cc-pVTZ waters the split form is 11 to 160 times as fast as the
+    // ordinary one for 300 quartets and, just below the line of 18,944, still 1.4 to 80 times ((dd|ps) at 4.04
+    // pairs 154 / 219 us, (pp|pp) 83 / 283, (ss|ss) of cc-pVDZ 57 / 4590).
     bool Engine::splitStore(const DevPairClass &bra, const DevPairClass &ket, long long n) const
     {
         const double k = (double)bra.n_ppairs / std::max<size_t>(bra.n_pairs, 1) * (double)ket.n_ppairs /

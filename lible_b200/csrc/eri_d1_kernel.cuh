@@ -784,11 +784,10 @@ namespace lible_b200
         // admits, at no fewer than 128 registers per thread
         static constexpr int MINB0 = (int)perSM(smem) < 65536 / (G * 128) ? (int)perSM(smem) : 65536 / (G * 128);
         static constexpr int MINB = MINB0 < 1 ? 1 : MINB0;
-        // the classes this form serves, as measured on the (H2O)_8 cc-pVTZ gradient: not a register
-        // class, a ket of at least S_cd = 5 spherical and H_cd = 10 Hermite functions (with smaller
-        // kets the W products are too thin to pay for the GE products and the staging; (dd|ss), (fp|ss)
-        // and (dd|ps) ran up to 2.3x slower than in the block form), and a layout that fits one block
-        // per SM
+        // the classes this form can serve: not a register class, a ket of at least S_cd = 5 spherical and
+        // H_cd = 10 Hermite functions (with smaller kets the W products are too thin to pay for the GE
+        // products and the staging), and a layout that fits one block per SM.  Those of them that
+        // d1WarpClass names run in the warp form instead (launchD1)
         static constexpr bool USE = !d1RegisterClass(LA, LB, LC, LD) && C::SCD >= 5 && C::HCD >= 10 &&
                                     smem1 <= 200 * 1024;
     };

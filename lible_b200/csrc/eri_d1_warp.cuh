@@ -13,6 +13,8 @@
 // warp in its own shared memory (warpHermiteR), so nothing synchronises more than one warp, the ket's E
 // and E1 are staged there with the four values of an element side by side, and the nine sums are
 // reduced once per quartet.
+// Bound by L1/TEX wavefronts (four R values and an index per Hermite pair, the ket tile): 71% of the unit on
+// (dp|ps) and (fd|ps) of (H2O)_4 cc-pVTZ, at 12 warps an SM of 164-168 registers, the FP64 pipe 32% active.
 #pragma once
 
 #include "eri_d1_kernel.cuh"

@@ -107,8 +107,9 @@ namespace lible_b200
     // Gamma-weighted bra matrices (4 x S_cd values each) stay within 72 doubles.  Kernel times of the
     // (H2O)_8 cc-pVTZ gradient against the block, tensor-pipe or register form that served the class:
     // (fd|ps) 26.1 -> 3.5 ms, (dd|ps) 22.6 -> 6.3, (fp|ps) 20.6 -> 6.2, (dd|ds) 14.5 -> 5.7,
-    // (dd|pp) 9.9 -> 4.9, (dp|pp) 16.3 -> 10.7, (dp|dp) 13.6 -> 9.0, (dp|ps) 17.3 -> 16.4; the whole
-    // gradient 437 -> 280 ms.  (fs) bras under thinner kets stay on the register form ((fs|ps) 5.4 ms).
+    // (dd|pp) 9.9 -> 4.9, (dp|pp) 16.3 -> 10.7, (dp|dp) 13.6 -> 9.0, (dp|ps) 17.3 -> 16.4; all launches
+    // 437 -> 280 ms, the gradient call 413 -> 265 ms.  With auxiliary shells, RI-J gradient of (H2O)_8 cc-pVTZ with
+    // def2-qzvp-rifit: 44.7 -> 27.9 ms of kernels, no class slower ((gs|gs) 47 -> 39 us, (hs|gs) 36 -> 34).  (fs) bras under thinner kets stay on the register form ((fs|ps) 5.4 ms).
     LB_HD constexpr bool d1WarpClass(int la, int lb, int lc, int ld)
     {
         const int hab = nherm(la + lb), scd = nsph(lc) * nsph(ld);
